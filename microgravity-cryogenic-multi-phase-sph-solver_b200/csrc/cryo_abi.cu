@@ -173,51 +173,43 @@ void cryo_ctx::configure_grid(const float* lo, const float* hi) {
   P.slab_z0 = 0;
   P.slab_z1 = P.nz;
   P.inv_cell = 1.0f / cell;
-  int bits = 0;
-  while (bits < 32 && ((uint64_t)1 << bits) <= (uint64_t)P.num_cells) ++bits;  // sentinel fits
-  P.key_bits = std::max(bits, 1);
   if (cell_cap < P.num_cells + 2) {
     if (cell_begin) CK(cudaFree(cell_begin));
     if (cell_fluid) CK(cudaFree(cell_fluid));
-    CK(cudaMalloc(&cell_begin, (size_t)(P.num_cells + 2) * sizeof(int)));
-    CK(cudaMalloc(&cell_fluid, (size_t)(P.num_cells + 2)));
-    cell_cap = P.num_cells + 2;
+    if (cell_work) CK(cudaFree(cell_work));
+    cell_begin = cell_work = nullptr;
+    cell_fluid = nullptr;
+    cell_cap = 0;
+    const size_t cap = ((size_t)P.num_cells + 2 + 7) / 8 * 8;  // k_cell_scan takes eight cells per thread
+    CK(cudaMalloc(&cell_begin, cap * sizeof(int)));
+    CK(cudaMalloc(&cell_fluid, cap));
+    CK(cudaMalloc(&cell_work, (2 * cap + cap / kScanCells + 2) * sizeof(int)));
+    cell_cap = (int)cap;
   }
+  CK(cudaMemsetAsync(cell_work, 0, (size_t)cell_cap * sizeof(int), stream));  // the counts
   CK(cudaMemsetAsync(cell_begin, 0, (size_t)(P.num_cells + 2) * sizeof(int), stream));
 }
 
-// Keys of the current positions in keys_a, then sort, cell table and gather
+// Keys of the current positions, then sort, cell table and gather
 // (SpatialHash::build, spatial_hash.cu:48-114).  Flips `cur`.
 void cryo_ctx::grid_build(int src) {
   const int G = grid_blocks();
-  LAUNCH(k_keys, G, kBlock, P, view(src), keys_a);
+  LAUNCH(k_keys, G, kBlock, P, view(src), cell_sort());
   sort_and_gather(src, LISTS_PHASE);
 }
 
-// Radix sort of keys_a, cell table, reorder gather into the other set and
+// Sort by the counted keys, cell table, reorder gather into the other set and
 // (with lists on) the neighbour / phase lists of the new order.
 void cryo_ctx::sort_and_gather(int src, int list_mode, bool reset_maxima) {
   const int G = grid_blocks();
-  const int tiles = (capacity + RS_TILE - 1) / RS_TILE;
-  const uint32_t* kin = keys_a;
-  const uint32_t* vin = nullptr;
-  uint32_t* kout = keys_b;
-  uint32_t* vout = vals_b;
-  for (int shift = 0; shift < P.key_bits; shift += RS_BITS) {
-    const int bits = std::min(RS_BITS, P.key_bits - shift);
-    LAUNCH(k_rs_upsweep, tiles, RS_THREADS, kin, shift, bits, dyn, hist);
-    LAUNCH(k_rs_scan, RS_BINS, RS_SCAN_THREADS, hist, dyn);
-    LAUNCH(k_rs_downsweep, tiles, RS_THREADS, kin, vin, kout, vout, shift, bits, dyn, hist);
-    kin = kout;
-    vin = vout;
-    kout = (kout == keys_b) ? keys_a : keys_b;
-    vout = (vout == vals_b) ? vals_a : vals_b;
-  }
-  sorted_keys = kin;
-  sorted_perm = vin;
-  LAUNCH(k_cells, G, kBlock, P, kin, dyn, cell_begin);
-  if (P.use_lists) CK(cudaMemsetAsync(cell_fluid, 0, (size_t)P.num_cells, stream));
-  LAUNCH(k_gather, G, kBlock, P, view(src), view(1 - src), vin, reduce(), reset_maxima ? 1 : 0);
+  const CellSort S = cell_sort();
+  const int scans = std::min((P.num_cells + kScanCells) / kScanCells, sm_count * 8);
+  LAUNCH(k_cell_scan, scans, kScanThreads, P, S, cell_fluid, ticket);
+  LAUNCH(k_cell_scatter, G, kBlock, P, S, dyn, cell_begin);
+  LAUNCH(k_cell_order, G, kBlock, P, S, dyn, cell_begin);
+  sorted_keys = S.sorted_key;
+  sorted_perm = S.perm;
+  LAUNCH(k_gather, G, kBlock, P, view(src), view(1 - src), S.perm, reduce(), reset_maxima ? 1 : 0);
   if (P.use_lists) {
     LAUNCH(k_build_lists, G, kBlock, P, view(1 - src), reduce(), list_mode);
     lists_built = true;
@@ -309,7 +301,7 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   // the step size, the frame and the kick-drift in one launch; the maxima
   // are reset by the gather
-  LAUNCH(k_begin_kick_drift_keys, G, kBlock, P, view(s), keys_a);
+  LAUNCH(k_begin_kick_drift_keys, G, kBlock, P, view(s), cell_sort());
   sort_and_gather(s, LISTS_PHASE, true);
   const int d = 1 - s;
   const View V = view(d);

@@ -113,7 +113,7 @@ struct Params {
   float f_rho_l, f_rho_v, f_T_sat, f_p_sat, f_R_gas, f_h_fg;
   // grid
   float ox, oy, oz, inv_cell, cell;
-  int nx, ny, nz, num_cells, key_bits;
+  int nx, ny, nz, num_cells;
   // neighbour lists (0: every pass scans the 27 cells)
   int use_lists;
   // 1: this context is one slab of a decomposed tank; the heat normalisation

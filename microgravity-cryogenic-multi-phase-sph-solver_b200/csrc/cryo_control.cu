@@ -84,7 +84,7 @@ __global__ void k_begin_step(Params P, View V, int mode) {
 // it and moves the manoeuvre frame to the new time level.  The maxima are
 // reset later in the step (k_gather with reset_maxima), once no block of this
 // kernel can still read them; the frame is not read here.
-__global__ void __launch_bounds__(kBlock) k_begin_kick_drift_keys(Params P, View V, uint32_t* __restrict__ keys) {
+__global__ void __launch_bounds__(kBlock) k_begin_kick_drift_keys(Params P, View V, CellSort S) {
   __shared__ float sdt;
   DynState* d = V.dyn;
   if (threadIdx.x == 0) {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kBlock) k_begin_kick_drift_keys(Params P, View
     float4 xp = V.xp[i];
     const int ph = ph_of(xp);
     if (is_fluid(ph)) kick_drift_one(P, V, i, dt, continuity, P.tvf, xp);
-    keys[i] = ph == kDead ? (uint32_t)P.num_cells : (uint32_t)cell_index(P, xyz(xp));
+    count_key(S, i, ph == kDead ? (uint32_t)P.num_cells : (uint32_t)cell_index(P, xyz(xp)));
   }
 }
 

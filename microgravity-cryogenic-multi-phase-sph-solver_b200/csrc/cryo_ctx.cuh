@@ -92,8 +92,6 @@ inline size_t particle_bytes(size_t cap) {
   for (int s = 0; s < 2; ++s) t += 5 * r(cap * 16) + r(cap * 4);    // persistent sets
   t += 8 * r(cap * 16) + 4 * r(cap * 4);                            // scratch
   t += 5 * r(cap * 4);                                              // sort keys/vals, split flags
-  const size_t tiles = (cap + RS_TILE - 1) / RS_TILE + 1;
-  t += r((tiles + 1) * RS_BINS * 4);                                // radix histogram + digit totals
   const size_t chunks = cap / kChunk + 2;
   t += r(chunks * 32 * 8);                                          // reduction partials
   t += r(64 * 8) + r(64);                                           // diagnostics out, tickets
@@ -151,7 +149,6 @@ struct cryo_ctx {
          *pc = nullptr, *aux = nullptr;
   float *rmin = nullptr, *wall_w = nullptr, *heat_w = nullptr, *nu_t = nullptr;
   uint32_t *keys_a = nullptr, *keys_b = nullptr, *vals_a = nullptr, *vals_b = nullptr, *split_flag = nullptr;
-  uint32_t* hist = nullptr;
   int *nbr = nullptr, *nbr_cnt = nullptr, *fluid_idx = nullptr, *wall_idx = nullptr;
   double* partials = nullptr;
   int max_chunks = 0;
@@ -164,6 +161,7 @@ struct cryo_ctx {
   // grid
   int* cell_begin = nullptr;
   uint8_t* cell_fluid = nullptr;  // 1: a fluid particle was sorted into the cell
+  int* cell_work = nullptr;  // the sort's counts, block prefixes and block totals (CellSort)
   int cell_cap = 0;
 
   // scalar block
@@ -340,6 +338,7 @@ struct cryo_ctx {
     arena.release();
     if (cell_begin) cudaFree(cell_begin);
     if (cell_fluid) cudaFree(cell_fluid);
+    if (cell_work) cudaFree(cell_work);
     if (dyn) cudaFree(dyn);
     if (hdyn) cudaFreeHost(hdyn);
     if (diag_host) cudaFreeHost(diag_host);
@@ -377,6 +376,9 @@ struct cryo_ctx {
     V.tape = tape_sums;
     V.tape_n = tape_n;
     return V;
+  }
+  CellSort cell_sort() const {
+    return CellSort{keys_a, vals_a, keys_b, vals_b, vals_a, cell_work, cell_work + cell_cap, cell_work + 2 * (size_t)cell_cap};
   }
   Reduce reduce() const { return Reduce{partials, ticket, max_chunks}; }
   // Particles the launch grids are sized for (0: the capacity).  Every step
@@ -457,8 +459,6 @@ struct cryo_ctx {
     uint32_t* nka = a.take<uint32_t>(cap); uint32_t* nkb = a.take<uint32_t>(cap);
     uint32_t* nva = a.take<uint32_t>(cap); uint32_t* nvb = a.take<uint32_t>(cap);
     uint32_t* nsf = a.take<uint32_t>(cap);
-    const size_t tiles = (size_t)(cap + RS_TILE - 1) / RS_TILE + 1;
-    uint32_t* nhist = a.take<uint32_t>(tiles * RS_BINS + RS_BINS);
     const int nchunks = cap / kChunk + 2;
     double* npart = a.take<double>((size_t)nchunks * 32);
     double* ndiag = a.take<double>(64);
@@ -490,7 +490,7 @@ struct cryo_ctx {
     a4 = na4; ab4 = nab4; fw = nfw; mw = nmw; vwp = nvwp; ns4 = nns4; pc = npc; aux = naux;
     rmin = nrmin; wall_w = nwall; heat_w = nheat; nu_t = nnut;
     keys_a = nka; keys_b = nkb; vals_a = nva; vals_b = nvb; split_flag = nsf;
-    hist = nhist; partials = npart; max_chunks = nchunks; diag_out = ndiag; ticket = ntick;
+    partials = npart; max_chunks = nchunks; diag_out = ndiag; ticket = ntick;
     nbr = nnbr; nbr_cnt = nnc; fluid_idx = nfi; wall_idx = nwi;
     lists_built = false;
     sorted_keys = nullptr;
@@ -511,7 +511,7 @@ struct cryo_ctx {
 
   // ------------------------------------------------------ step pieces
   void grid_build(int src);               // keys of current positions, sort, cells, gather, lists
-  void sort_and_gather(int src, int list_mode, bool reset_maxima = false);  // after keys_a holds the keys
+  void sort_and_gather(int src, int list_mode, bool reset_maxima = false);  // after the keys are counted
   void evaluate_rates(int s, bool maxima_reset, bool density_done, bool tape = false);
   void enqueue_step(int s, const StepTape* tape = nullptr);
   void launch_step();

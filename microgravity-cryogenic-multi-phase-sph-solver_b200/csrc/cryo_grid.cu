@@ -1,204 +1,129 @@
 // cryo_grid.cu -- uniform-grid neighbour search on the GPU: integer cell keys,
-// a stable LSD radix sort, the dense cell table and the reorder gather.
+// a stable counting sort by cell, the dense cell table and the reorder gather.
 // Replaces SpatialHash::build / reorder_particles (spatial_hash.cu:48-138).
 #include "cryo_kernels.cuh"
 
 namespace cryo {
 
-// Keys and the identity permutation (spatial_hash.cu:61-68): dead particles
-// get the sentinel num_cells so they sort to the end.
-__global__ void k_keys(Params P, View V, uint32_t* __restrict__ keys) {
+// Cell keys (spatial_hash.cu:61-68): dead particles get the sentinel
+// num_cells so they sort to the end.
+__global__ void k_keys(Params P, View V, CellSort S) {
   const int n = V.dyn->n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 xp = V.xp[i];
-    keys[i] = ph_of(xp) == kDead ? (uint32_t)P.num_cells : (uint32_t)cell_index(P, xyz(xp));
+    count_key(S, i, ph_of(xp) == kDead ? (uint32_t)P.num_cells : (uint32_t)cell_index(P, xyz(xp)));
   }
 }
 
-// ---------------------------------------------------------------- radix sort
-// Stable LSD radix sort of (key, value) pairs, RS_BITS-wide digits.  One
-// tile of RS_TILE keys per block; blocks beyond ceil(n / RS_TILE) exit, so the
-// grid can be sized from the capacity and the key count stays on the device.
-// Per pass: upsweep (digit histogram per tile), scan (digit-major, tile-minor
-// exclusive scan), downsweep (stable in-tile ranking with warp match_any,
-// scatter).  No atomics decide positions, so the permutation is unique.
-
-__global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const uint32_t* __restrict__ keys, int shift, int bits,
-                                                           const DynState* __restrict__ dyn,
-                                                           uint32_t* __restrict__ hist) {
-  const int n = dyn->n;
-  const int nt = (n + RS_TILE - 1) / RS_TILE;
-  const int b = blockIdx.x;
-  if (b >= nt) return;
-  __shared__ uint32_t cnt[RS_BINS];
-  for (int d = threadIdx.x; d < RS_BINS; d += blockDim.x) cnt[d] = 0;
-  __syncthreads();
-  const uint32_t mask = (1u << bits) - 1u;
-  const int base = b * RS_TILE;
-  for (int k = threadIdx.x; k < RS_TILE; k += blockDim.x) {
-    const int idx = base + k;
-    if (idx < n) atomicAdd(&cnt[(keys[idx] >> shift) & mask], 1u);
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < RS_BINS; d += blockDim.x) hist[d * nt + b] = cnt[d];
-}
-
-// Per digit (one block each): exclusive scan of the tile counts hist[d][*]
-// in place and the digit total in hist_tot[d].  The downsweep adds the
-// exclusive prefix of the digit totals.
-__global__ void __launch_bounds__(RS_SCAN_THREADS) k_rs_scan(uint32_t* __restrict__ hist,
-                                                              const DynState* __restrict__ dyn) {
-  const int n = dyn->n;
-  const int nt = (n + RS_TILE - 1) / RS_TILE;
-  const int d = blockIdx.x;
-  uint32_t* row = hist + (size_t)d * nt;
-  const int per = (nt + blockDim.x - 1) / blockDim.x;
-  const int lo = threadIdx.x * per, hi = min(lo + per, nt);
-  uint32_t s = 0;
-  for (int k = lo; k < hi; ++k) s += row[k];
-  __shared__ uint32_t warp_tot[32];
+// ------------------------------------------------------------- cell sort
+// The stable sort by cell key as a counting sort over the dense cells, whose
+// prefix sums are the cell table the passes need anyway:
+//   1. the key kernel counts the particles of every cell and notes which
+//      number each particle drew (the order of the draws is arbitrary);
+//   2. k_cell_scan: exclusive prefix sums of the counts, kScanCells cells per
+//      block, and (last block) of the blocks' totals;
+//   3. k_cell_scatter: particle index and key to the cell's range, in drawn
+//      order; the finished cell table;
+//   4. k_cell_order: inside its cell a particle's place is the number of
+//      smaller indices there, which makes the result the stable sort whatever
+//      the draws were.
+// Three launches whatever the number of cells (the radix sort before it took
+// three per 8-bit digit and a fourth kind for the table).  A tank's cell holds
+// about 18 particles, so step 4 reads one or two cache lines per particle.
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(Params P, CellSort S, uint8_t* __restrict__ cell_fluid,
+                                                            unsigned* ticket) {
+  constexpr int kPer = kScanCells / kScanThreads;
+  static_assert(kPer == 8, "8 cells per thread");
+  __shared__ int wtot[kScanThreads / 32];
+  const int cells = P.num_cells + 1;  // the sentinel too
+  const int blocks = (cells + kScanCells - 1) / kScanCells;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t incl = s;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : 0;
+  // exclusive prefix of one value per thread over the block; `total` to all
+  auto block_scan = [&](int v, int& total) {
+    int incl = v;
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += t;
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
     }
-    warp_tot[lane] = w;  // inclusive over warps
-  }
-  __syncthreads();
-  uint32_t run = (incl - s) + (warp > 0 ? warp_tot[warp - 1] : 0);
-  for (int k = lo; k < hi; ++k) {
-    const uint32_t c = row[k];
-    row[k] = run;
-    run += c;
-  }
-  if (threadIdx.x == blockDim.x - 1) hist[(size_t)RS_BINS * nt + d] = run;  // digit total
-}
-
-__global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const uint32_t* __restrict__ kin,
-                                                             const uint32_t* __restrict__ vin,
-                                                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                             int shift, int bits, const DynState* __restrict__ dyn,
-                                                             const uint32_t* __restrict__ hist) {
-  const int n = dyn->n;
-  const int nt = (n + RS_TILE - 1) / RS_TILE;
-  const int b = blockIdx.x;
-  if (b >= nt) return;
-  constexpr int kWarps = RS_THREADS / 32;
-  constexpr int kPer = RS_TILE / kWarps / 32;  // keys per lane
-  __shared__ uint32_t wcnt[kWarps][RS_BINS];
-  for (int t = threadIdx.x; t < kWarps * RS_BINS; t += blockDim.x) (&wcnt[0][0])[t] = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t mask = (1u << bits) - 1u;
-  const int wbase = b * RS_TILE + warp * (kPer * 32);
-  uint32_t key[kPer], val[kPer], rank[kPer];
+    if (lane == 31) wtot[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int idx = wbase + k * 32 + lane;
-    const bool valid = idx < n;
-    key[k] = valid ? kin[idx] : 0u;
-    val[k] = valid ? (vin ? vin[idx] : (uint32_t)idx) : 0u;
-    const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
-    const uint32_t d = (key[k] >> shift) & mask;
-    rank[k] = 0;
-    if (valid) {
-      const uint32_t peers = __match_any_sync(vmask, d);
-      const uint32_t before = wcnt[warp][d];
-      const int leader = __ffs(peers) - 1;
-      rank[k] = before + __popc(peers & lt_mask);
-      __syncwarp(vmask);
-      if (lane == leader) wcnt[warp][d] = before + __popc(peers);
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      const int t = wtot[w];
+      if (w < warp) before += t;
+      total += t;
     }
-    __syncwarp();
-  }
-  __syncthreads();
-  // digit offsets: exclusive scan of the digit totals (RS_BINS entries)
-  __shared__ uint32_t dig[RS_BINS];
-  for (int d = threadIdx.x; d < RS_BINS; d += blockDim.x) dig[d] = hist[(size_t)RS_BINS * nt + d];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t carry = 0;
-    for (int base = 0; base < RS_BINS; base += 32) {
-      const uint32_t x = dig[base + threadIdx.x];
-      uint32_t incl = x;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (threadIdx.x >= o) incl += t;
+    __syncthreads();
+    return before + incl - v;
+  };
+  for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
+    // the arrays hold a multiple of kPer entries, zero beyond the last cell
+    const int base = b * kScanCells + threadIdx.x * kPer;
+    int c[kPer], sum = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; q += 4) {
+      const int4 v = base < cells ? *reinterpret_cast<const int4*>(S.count + base + q) : make_int4(0, 0, 0, 0);
+      c[q] = v.x; c[q + 1] = v.y; c[q + 2] = v.z; c[q + 3] = v.w;
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) sum += c[q];
+    int total;
+    int run = block_scan(sum, total);
+    if (base < cells) {
+#pragma unroll
+      for (int q = 0; q < kPer; q += 4) {
+        int4 v;
+        v.x = run; v.y = v.x + c[q]; v.z = v.y + c[q + 1]; v.w = v.z + c[q + 2];
+        run = v.w + c[q + 3];
+        *reinterpret_cast<int4*>(S.local + base + q) = v;
+        *reinterpret_cast<int4*>(S.count + base + q) = make_int4(0, 0, 0, 0);  // ready for the next build
       }
-      dig[base + threadIdx.x] = carry + incl - x;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
+      if (P.use_lists) *reinterpret_cast<uint2*>(cell_fluid + base) = make_uint2(0u, 0u);
     }
+    if (threadIdx.x == 0) S.sums[b] = total;
   }
-  __syncthreads();
-  // exclusive scan of the per-warp counts across warps, per digit
-  for (int d = threadIdx.x; d < RS_BINS; d += blockDim.x) {
-    uint32_t run = dig[d] + hist[d * nt + b];
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const uint32_t c = wcnt[w][d];
-      wcnt[w][d] = run;
-      run += c;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int idx = wbase + k * 32 + lane;
-    if (idx < n) {
-      const uint32_t d = (key[k] >> shift) & mask;
-      const uint32_t pos = wcnt[warp][d] + rank[k];
-      kout[pos] = key[k];
-      vout[pos] = val[k];
+  if (last_block(ticket)) {
+    int carry = 0;
+    for (int b0 = 0; b0 < blocks; b0 += kScanThreads) {
+      const int b = b0 + threadIdx.x;
+      const int v = b < blocks ? __ldcg(S.sums + b) : 0;
+      int total;
+      const int pre = block_scan(v, total);
+      if (b < blocks) S.sums[b] = carry + pre;
+      carry += total;
     }
   }
 }
 
-// Dense cell table: cell_begin[c] = first sorted index with key >= c, for
-// c in [0, num_cells]; cell_begin[num_cells] = number of live particles.
-// One pass over the sorted keys (clamped to num_cells: dead particles carry
-// that sentinel) instead of a binary search per cell: position i (0..n, with
-// key[-1] = -1 and key[n] = num_cells) writes i to every cell in
-// (key[i-1], key[i]], so each cell receives its lower bound exactly once.
-// A run longer than 8 cells (the empty cells of padding layers or around a
-// tank) is written by the whole warp together.
-__global__ void k_cells(Params P, const uint32_t* __restrict__ keys, DynState* dyn, int* __restrict__ cell_begin) {
-  const int n = dyn->n;
-  const int nc = P.num_cells;
-  const int lane = threadIdx.x & 31;
-  // whole warps walk 32 positions at a time (a warp-uniform loop), so every
-  // lane takes part in the ballots
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 <= n; w += warps) {
-    const int i = w * 32 + lane;
-    int lo = 0, hi = -1;  // cells lo..hi get i
-    if (i <= n) {
-      lo = (i == 0 ? -1 : (int)min(__ldg(keys + i - 1), (uint32_t)nc)) + 1;
-      hi = i == n ? nc : (int)min(__ldg(keys + i), (uint32_t)nc);
-    }
-    const int len = hi - lo + 1;
-    if (len > 0 && len <= 8) {
-      for (int c = lo; c <= hi; ++c) cell_begin[c] = i;
-      if (hi == nc) dyn->n_alive = i;
-    }
-    unsigned longs = __ballot_sync(0xffffffffu, len > 8);
-    while (longs) {
-      const int src = __ffs(longs) - 1;
-      longs &= longs - 1u;
-      const int rl = __shfl_sync(0xffffffffu, lo, src), rh = __shfl_sync(0xffffffffu, hi, src);
-      const int ri = __shfl_sync(0xffffffffu, i, src);
-      for (int c = rl + lane; c <= rh; c += 32) cell_begin[c] = ri;
-      if (lane == src && rh == nc) dyn->n_alive = ri;
-    }
+__global__ void __launch_bounds__(kBlock) k_cell_scatter(Params P, CellSort S, DynState* dyn,
+                                                         int* __restrict__ cell_begin) {
+  const int n = dyn->n, nc = P.num_cells;
+  const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int i = first; i < n; i += step) {
+    const uint32_t key = S.key[i];
+    const int at = S.local[key] + S.sums[key / kScanCells] + (int)S.slot[i];
+    S.drawn[at] = (uint32_t)i;
+    S.sorted_key[at] = key;
+  }
+  for (int c = first; c <= nc; c += step) {
+    const int b = S.local[c] + S.sums[c / kScanCells];
+    cell_begin[c] = b;
+    if (c == nc) dyn->n_alive = b;
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) k_cell_order(Params P, CellSort S, const DynState* __restrict__ dyn,
+                                                       const int* __restrict__ cell_begin) {
+  const int n = dyn->n_alive;  // the dead are dropped by the gather
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    const uint32_t key = S.sorted_key[p];
+    const uint32_t i = S.drawn[p];
+    const int b = __ldg(cell_begin + key), e = __ldg(cell_begin + key + 1);
+    int smaller = 0;
+    for (int q = b; q < e; ++q) smaller += __ldg(S.drawn + q) < i;
+    S.perm[b + smaller] = i;
   }
 }
 

@@ -6,14 +6,28 @@
 
 namespace cryo {
 
-constexpr int RS_THREADS = 256;
-#ifndef RS_TILE_KEYS
-#define RS_TILE_KEYS 1024
-#endif
-constexpr int RS_TILE = RS_TILE_KEYS;  // keys per radix tile (RS_TILE / RS_THREADS per thread)
-constexpr int RS_BITS = 8;
-constexpr int RS_BINS = 1 << RS_BITS;
-constexpr int RS_SCAN_THREADS = 256;
+// Cells per block of the cell-table scan.
+constexpr int kScanThreads = 256;
+constexpr int kScanCells = 2048;
+
+// Arrays of the sort by cell key (cryo_grid.cu).
+struct CellSort {
+  uint32_t *key, *slot;          // per particle: its cell, its number among the cell's draws
+  uint32_t *sorted_key, *drawn;  // per sorted place: the cell, the particle in drawn order
+  uint32_t* perm;                // per sorted place: the particle of the stable sort (reuses slot's storage)
+  int *count, *local, *sums;     // per cell: particles (zero between builds), prefix in its block; per block: prefix
+};
+// Key of particle i, counted: lanes of the warp that share a cell draw their
+// numbers with one atomic (neighbours in the previous order mostly do).
+__device__ inline void count_key(const CellSort& S, int i, uint32_t key) {
+  const unsigned peers = __match_any_sync(__activemask(), key);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(S.count + key, __popc(peers));
+  base = __shfl_sync(peers, base, leader);
+  S.key[i] = key;
+  S.slot[i] = (uint32_t)(base + __popc(peers & ((1u << lane) - 1u)));
+}
 
 // Layout of the FP64 partials of one reduction: partials[v * max_chunks + c].
 struct Reduce {
@@ -176,12 +190,10 @@ __device__ inline void publish_chunk(const Reduce& R, int c, double (&v)[NV], do
 __device__ inline int num_chunks(int n) { return (n + kChunk - 1) / kChunk; }
 
 // grid (cryo_grid.cu)
-__global__ void k_keys(Params P, View V, uint32_t* keys);
-__global__ void k_rs_upsweep(const uint32_t* keys, int shift, int bits, const DynState* dyn, uint32_t* hist);
-__global__ void k_rs_scan(uint32_t* hist, const DynState* dyn);
-__global__ void k_rs_downsweep(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int shift,
-                               int bits, const DynState* dyn, const uint32_t* hist);
-__global__ void k_cells(Params P, const uint32_t* keys, DynState* dyn, int* cell_begin);
+__global__ void k_keys(Params P, View V, CellSort S);
+__global__ void k_cell_scan(Params P, CellSort S, uint8_t* cell_fluid, unsigned* ticket);
+__global__ void k_cell_scatter(Params P, CellSort S, DynState* dyn, int* cell_begin);
+__global__ void k_cell_order(Params P, CellSort S, const DynState* dyn, const int* cell_begin);
 __global__ void k_gather(Params P, View src, View dst, const uint32_t* perm, Reduce R, int reset_maxima);
 enum { LISTS_ONLY = 0, LISTS_PHASE = 1 };
 __global__ void k_build_lists(Params P, View V, Reduce R, int mode);
@@ -301,7 +313,7 @@ __device__ inline void saturation_update(const Params& P, DynState* d, bool clos
   }
 }
 __global__ void k_saturation(Params P, View V, Reduce R, int end_of_step);
-__global__ void k_begin_kick_drift_keys(Params P, View V, uint32_t* keys);
+__global__ void k_begin_kick_drift_keys(Params P, View V, CellSort S);
 __global__ void k_kick_saturation(Params P, View V, Reduce R);
 __global__ void k_diagnostics(Params P, View V, Reduce R, double* out);
 
