@@ -175,15 +175,13 @@ void cryo_ctx::configure_grid(const float* lo, const float* hi) {
   P.inv_cell = 1.0f / cell;
   if (cell_cap < P.num_cells + 2) {
     if (cell_begin) CK(cudaFree(cell_begin));
-    if (cell_fluid) CK(cudaFree(cell_fluid));
-    if (cell_work) CK(cudaFree(cell_work));
-    cell_begin = cell_work = nullptr;
-    cell_fluid = nullptr;
+    cell_begin = nullptr;
     cell_cap = 0;
     const size_t cap = ((size_t)P.num_cells + 2 + 7) / 8 * 8;  // k_cell_scan takes eight cells per thread
-    CK(cudaMalloc(&cell_begin, cap * sizeof(int)));
-    CK(cudaMalloc(&cell_fluid, cap));
-    CK(cudaMalloc(&cell_work, (2 * cap + cap / kScanCells + 2) * sizeof(int)));
+    // table, kinds, counts and block prefixes (cap entries each), block totals
+    CK(cudaMalloc(&cell_begin, (4 * cap + cap / kScanCells + 2) * sizeof(int)));
+    cell_kinds = reinterpret_cast<uint32_t*>(cell_begin + cap);
+    cell_work = cell_begin + 2 * cap;
     cell_cap = (int)cap;
   }
   CK(cudaMemsetAsync(cell_work, 0, (size_t)cell_cap * sizeof(int), stream));  // the counts
@@ -204,16 +202,23 @@ void cryo_ctx::sort_and_gather(int src, int list_mode, bool reset_maxima) {
   const int G = grid_blocks();
   const CellSort S = cell_sort();
   const int scans = std::min((P.num_cells + kScanCells) / kScanCells, sm_count * 8);
-  LAUNCH(k_cell_scan, scans, kScanThreads, P, S, cell_fluid, ticket);
+  LAUNCH(k_cell_scan, scans, kScanThreads, P, S, cell_kinds, ticket);
   LAUNCH(k_cell_scatter, G, kBlock, P, S, dyn, cell_begin);
   LAUNCH(k_cell_order, G, kBlock, P, S, dyn, cell_begin);
   sorted_keys = S.sorted_key;
   sorted_perm = S.perm;
-  LAUNCH(k_gather, G, kBlock, P, view(src), view(1 - src), S.perm, reduce(), reset_maxima ? 1 : 0);
+  LAUNCH(k_gather, G, kBlock, P, view(src), view(1 - src), S.perm, S.sorted_key, reduce(), reset_maxima ? 1 : 0);
   if (P.use_lists) {
-    LAUNCH(k_build_lists, G, kBlock, P, view(1 - src), reduce(), list_mode);
+    build_lists(view(1 - src), list_mode);
     lists_built = true;
   }
+}
+
+void cryo_ctx::build_lists(const View& V, int mode) {
+  if (loaded_n <= LIST_LANES_MAX)
+    LAUNCH(k_build_lists<LIST_LANES>, list_blocks(LIST_LANES), kBlock, P, V, reduce(), mode);
+  else
+    LAUNCH(k_build_lists<1>, list_blocks(1), kBlock, P, V, reduce(), mode);
 }
 
 // Solver::evaluate_rates (sph_solver.cu:449-480) on set s.  density_done:
@@ -228,8 +233,10 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
   }
   FIELD_LAUNCH(k_wall, G, kBlock, P, V);
   slab_point(SLAB_HALO, s);
-  if (tape) FIELD_LAUNCH(k_interface<1>, G, kBlock, P, V, reduce(), P.thermal ? 1 : 0);
-  else FIELD_LAUNCH(k_interface<0>, G, kBlock, P, V, reduce(), P.thermal ? 1 : 0);
+  if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V);
+  else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V);
+  // without a heater there is nothing to normalise: the force pass reads a zero power
+  if (P.thermal && P.heat_power != 0.0f) LAUNCH(k_heat_sum, G, kBlock, P, V, reduce());
   slab_point(P.thermal ? SLAB_HEAT : SLAB_HALO, s);
   if (P.sps) {
     FIELD_LAUNCH(k_sps, G, kBlock, P, V);
@@ -326,7 +333,7 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
     slab_point(SLAB_HALO, d);
     // the phase-change passes search around the shifted positions
     // (old cell table), as for_each_neighbor does in the reference
-    if (P.use_lists) LAUNCH(k_build_lists, G, kBlock, P, V, reduce(), LISTS_ONLY);
+    if (P.use_lists) build_lists(V, LISTS_ONLY);
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
@@ -1467,7 +1474,7 @@ int cryo_pass(cryo_ctx* c, int pass) {
       case CRYO_PASS_NORMALIZE_MASSES: FIELD_KERNEL(c, k_normalize_masses)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_EOS: FIELD_KERNEL(c, k_eos)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_WALL_BOUNDARY: FIELD_KERNEL(c, k_wall)<<<G, kBlock, 0, st>>>(P, V); break;
-      case CRYO_PASS_INTERFACE: FIELD_KERNEL(c, k_interface<0>)<<<G, kBlock, 0, st>>>(P, V, R, 0); break;
+      case CRYO_PASS_INTERFACE: FIELD_KERNEL(c, k_interface<0>)<<<c->interface_blocks(), INTERFACE_BLOCK, 0, st>>>(P, V); break;
       case CRYO_PASS_TRANSPORT: FIELD_KERNEL(c, k_forces_t<-1>)<<<c->forces_blocks(), FORCES_BLOCK, 0, st>>>(P, V, FORCE_TRANSPORT); break;
       case CRYO_PASS_SPS: FIELD_KERNEL(c, k_sps)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_MOMENTUM: FIELD_KERNEL(c, k_forces_t<-1>)<<<c->forces_blocks(), FORCES_BLOCK, 0, st>>>(P, V, FORCE_MOMENTUM); break;
@@ -1491,7 +1498,7 @@ int cryo_pass(cryo_ctx* c, int pass) {
         LAUNCH_CHECK();
         FIELD_KERNEL(c, k_shift_apply)<<<G, kBlock, 0, st>>>(P, V);
         LAUNCH_CHECK();
-        if (P.use_lists) k_build_lists<<<G, kBlock, 0, st>>>(P, V, R, LISTS_ONLY);
+        if (P.use_lists) c->build_lists(V, LISTS_ONLY);
         break;
       case CRYO_PASS_PC_SOURCES: k_pc_sources<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_PC_NORMALIZE: k_pc_normalize<<<G, kBlock, 0, st>>>(P, V, R, 0); break;

@@ -33,6 +33,11 @@ constexpr float kPi = 3.14159265358979323846f;
 constexpr int kBlock = 256;      // threads per block of the particle kernels
 constexpr int kChunk = kBlock;   // particles per reduction partial (fixed tree, tank-local)
 
+// Bits of View::cell_kinds: one byte each, so that they can be set by plain stores.
+constexpr uint32_t kCellLiquid = 1u, kCellVapor = 1u << 8, kCellWall = 1u << 16, kCellNearSource = 1u << 24;
+// Bits of View::near_kinds.
+constexpr int kNearLiquid = 1, kNearVapor = 2, kNearWall = 4;
+
 __host__ __device__ inline bool is_fluid(int ph) { return ph <= kVapor; }
 __host__ __device__ inline int phase_index(int ph) { return ph == kVapor ? 1 : 0; }
 
@@ -222,7 +227,13 @@ struct View {
   // same operations (written by the density pass, valid until the kick)
   float4* aux;
   const int* cell_begin;  // dense cell prefix table, num_cells + 1 entries
-  uint8_t* cell_fluid;    // per cell: 1 if a fluid particle was sorted into it (lists mode)
+  // lists mode, per cell: what was sorted into it (kCellLiquid ...), and
+  // whether a cell of its 27 holds a phase-change source (kCellNearSource)
+  uint32_t* cell_kinds;
+  // lists mode, per particle: the kinds of all cells its neighbours can be in
+  // (set by the list build; a particle with no wall and none of the other
+  // phase around skips the interface pass)
+  uint8_t* near_kinds;
   DynState* dyn;
   // maneuver table
   const double* man_t;

@@ -233,6 +233,32 @@ __global__ void __launch_bounds__(kBlock) k_kick_saturation(Params P, View V, Re
   d->last_dt = (double)d->dt;
 }
 
+// The heat-weight normalisation of a step with a heater (sph_solver.cu:101-104,
+// 466-472): the FP64 sum of the fluid particles' heat weights, chunk by chunk
+// of the fluid list, after the interface pass.
+__global__ void __launch_bounds__(kBlock) k_heat_sum(Params P, View V, Reduce R) {
+  __shared__ double sh[kBlock / 32];
+  DynState* d = V.dyn;
+  const Range rg = fluid_range(P, V);
+  const int nch = num_chunks(rg.count);
+  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
+    const int t = c * kChunk + threadIdx.x;
+    double s[1] = {0.0};
+    if (t < rg.count) {
+      const int i = particle_at(rg, t);
+      if (is_fluid(ph_of(V.xp[i])) && owned(d->own_lo, d->own_hi, d->n_sorted, i)) s[0] = (double)V.heat_w[i];
+    }
+    publish_chunk<1>(R, c, s, sh);
+  }
+  if (last_block(R.ticket)) {
+    const double S = block_sum_partials(R, 0, nch);
+    if (threadIdx.x != 0) return;
+    d->heat_sum = S;
+    // the slabs set heat_inv_norm from their combined sums
+    if (!P.slab && d->thermal_on) d->heat_inv_norm = S > 0 ? (float)(1.0 / S) : 0.0f;
+  }
+}
+
 // Heat-weight normalisation on its own (sph_solver.cu:466-472), for
 // operator-level calls.
 __global__ void __launch_bounds__(kBlock) k_heat_norm(Params P, View V, Reduce R) {

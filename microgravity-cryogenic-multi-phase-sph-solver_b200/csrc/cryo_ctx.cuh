@@ -89,13 +89,14 @@ inline size_t particle_bytes(size_t cap) {
   const size_t a = 256;
   auto r = [&](size_t b) { return (b + a - 1) / a * a; };
   size_t t = 0;
-  for (int s = 0; s < 2; ++s) t += 5 * r(cap * 16) + r(cap * 4);    // persistent sets
+  for (int s = 0; s < 2; ++s) t += r((cap + kListPad) * 16) + 4 * r(cap * 16) + r(cap * 4);  // persistent sets
   t += 8 * r(cap * 16) + 4 * r(cap * 4);                            // scratch
   t += 5 * r(cap * 4);                                              // sort keys/vals, split flags
   const size_t chunks = cap / kChunk + 2;
   t += r(chunks * 32 * 8);                                          // reduction partials
   t += r(64 * 8) + r(64);                                           // diagnostics out, tickets
   t += r(cap * 4 * (size_t)kMaxNbr) + 3 * r(cap * 4);              // neighbour lists, counts, phase lists
+  t += r(cap);                                                      // kinds around each particle
   return t;
 }
 
@@ -150,6 +151,7 @@ struct cryo_ctx {
   float *rmin = nullptr, *wall_w = nullptr, *heat_w = nullptr, *nu_t = nullptr;
   uint32_t *keys_a = nullptr, *keys_b = nullptr, *vals_a = nullptr, *vals_b = nullptr, *split_flag = nullptr;
   int *nbr = nullptr, *nbr_cnt = nullptr, *fluid_idx = nullptr, *wall_idx = nullptr;
+  uint8_t* near_kinds = nullptr;
   double* partials = nullptr;
   int max_chunks = 0;
   double* diag_out = nullptr;
@@ -159,8 +161,8 @@ struct cryo_ctx {
   int last_sort_n = 0;
 
   // grid
-  int* cell_begin = nullptr;
-  uint8_t* cell_fluid = nullptr;  // 1: a fluid particle was sorted into the cell
+  int* cell_begin = nullptr;  // one allocation with the two below
+  uint32_t* cell_kinds = nullptr;  // View::cell_kinds
   int* cell_work = nullptr;  // the sort's counts, block prefixes and block totals (CellSort)
   int cell_cap = 0;
 
@@ -337,8 +339,6 @@ struct cryo_ctx {
     if (stream) cudaStreamSynchronize(stream);
     arena.release();
     if (cell_begin) cudaFree(cell_begin);
-    if (cell_fluid) cudaFree(cell_fluid);
-    if (cell_work) cudaFree(cell_work);
     if (dyn) cudaFree(dyn);
     if (hdyn) cudaFreeHost(hdyn);
     if (diag_host) cudaFreeHost(diag_host);
@@ -363,7 +363,8 @@ struct cryo_ctx {
     V.rmin = rmin; V.wall_w = wall_w; V.heat_w = heat_w; V.nu_t = nu_t;
     V.aux = aux;
     V.cell_begin = cell_begin;
-    V.cell_fluid = cell_fluid;
+    V.cell_kinds = cell_kinds;
+    V.near_kinds = near_kinds;
     V.dyn = dyn;
     V.man_t = man_t; V.man_acc = man_acc; V.man_omega = man_omega;
     V.partials = partials;
@@ -400,6 +401,10 @@ struct cryo_ctx {
     const int need = (span() + per_block - 1) / per_block;
     return std::max(1, std::min(need, sm_count * 8));
   }
+  int interface_blocks() const {
+    const int per_block = INTERFACE_BLOCK * grid_tile;
+    return std::max(1, (span() + per_block - 1) / per_block);
+  }
   // force pass: one thread per particle (times the tile) up to two
   // full-occupancy waves
   int forces_blocks() const {
@@ -407,6 +412,13 @@ struct cryo_ctx {
     const int need = (span() + per_block - 1) / per_block;
     return std::max(1, std::min(need, sm_count * (2048 / FORCES_BLOCK) * 2));
   }
+  // list build, L lanes per particle
+  int list_blocks(int L) const {
+    const int per_block = kBlock / L * grid_tile;
+    const int need = (span() + per_block - 1) / per_block;
+    return std::max(1, std::min(need, sm_count * 32));
+  }
+  void build_lists(const View& V, int mode);
   void invalidate_graphs() {
     ++generation;
     for (int k = 0; k < 2; ++k) {
@@ -447,7 +459,7 @@ struct cryo_ctx {
     CK(cudaMemsetAsync(a.base, 0, a.size, stream));
     Persist ns[2];
     for (int s = 0; s < 2; ++s) {
-      ns[s].xp = a.take<float4>(cap); ns[s].vT = a.take<float4>(cap); ns[s].vt = a.take<float4>(cap);
+      ns[s].xp = a.take<float4>((size_t)cap + kListPad); ns[s].vT = a.take<float4>(cap); ns[s].vt = a.take<float4>(cap);
       ns[s].nrm = a.take<float4>(cap); ns[s].mrps = a.take<float4>(cap); ns[s].id = a.take<uint32_t>(cap);
     }
     float4* na4 = a.take<float4>(cap); float4* nab4 = a.take<float4>(cap); float4* nfw = a.take<float4>(cap);
@@ -467,6 +479,7 @@ struct cryo_ctx {
     int* nnc = a.take<int>(cap);
     int* nfi = a.take<int>(cap);
     int* nwi = a.take<int>(cap);
+    uint8_t* nnk = a.take<uint8_t>(cap);
     if (a.used > a.size) throw std::runtime_error("internal: arena overflow");
     // keep the first n particles of every array (ParticleSystem::grow,
     // particle_system.cpp:66-71)
@@ -491,7 +504,7 @@ struct cryo_ctx {
     rmin = nrmin; wall_w = nwall; heat_w = nheat; nu_t = nnut;
     keys_a = nka; keys_b = nkb; vals_a = nva; vals_b = nvb; split_flag = nsf;
     partials = npart; max_chunks = nchunks; diag_out = ndiag; ticket = ntick;
-    nbr = nnbr; nbr_cnt = nnc; fluid_idx = nfi; wall_idx = nwi;
+    nbr = nnbr; nbr_cnt = nnc; fluid_idx = nfi; wall_idx = nwi; near_kinds = nnk;
     lists_built = false;
     sorted_keys = nullptr;
     sorted_perm = nullptr;

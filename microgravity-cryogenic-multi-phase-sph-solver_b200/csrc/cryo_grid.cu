@@ -1,6 +1,8 @@
 // cryo_grid.cu -- uniform-grid neighbour search on the GPU: integer cell keys,
 // a stable counting sort by cell, the dense cell table and the reorder gather.
 // Replaces SpatialHash::build / reorder_particles (spatial_hash.cu:48-138).
+#include <type_traits>
+
 #include "cryo_kernels.cuh"
 
 namespace cryo {
@@ -30,7 +32,7 @@ __global__ void k_keys(Params P, View V, CellSort S) {
 // Three launches whatever the number of cells (the radix sort before it took
 // three per 8-bit digit and a fourth kind for the table).  A tank's cell holds
 // about 18 particles, so step 4 reads one or two cache lines per particle.
-__global__ void __launch_bounds__(kScanThreads) k_cell_scan(Params P, CellSort S, uint8_t* __restrict__ cell_fluid,
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(Params P, CellSort S, uint32_t* __restrict__ cell_kinds,
                                                             unsigned* ticket) {
   constexpr int kPer = kScanCells / kScanThreads;
   static_assert(kPer == 8, "8 cells per thread");
@@ -79,8 +81,8 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Params P, CellSort S
         run = v.w + c[q + 3];
         *reinterpret_cast<int4*>(S.local + base + q) = v;
         *reinterpret_cast<int4*>(S.count + base + q) = make_int4(0, 0, 0, 0);  // ready for the next build
+        if (P.use_lists) *reinterpret_cast<uint4*>(cell_kinds + base + q) = make_uint4(0u, 0u, 0u, 0u);
       }
-      if (P.use_lists) *reinterpret_cast<uint2*>(cell_fluid + base) = make_uint2(0u, 0u);
     }
     if (threadIdx.x == 0) S.sums[b] = total;
   }
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_order(Params P, CellSort S, con
 // into the chunk offsets of the ordered phase index lists (partials rows 0
 // and 1) and their lengths.
 __global__ void __launch_bounds__(kBlock) k_gather(Params P, View src, View dst, const uint32_t* __restrict__ perm,
-                                                   Reduce R, int reset_maxima) {
+                                                   const uint32_t* __restrict__ cells, Reduce R, int reset_maxima) {
   __shared__ double sh[2 * kBlock / 32];
   DynState* dyn = src.dyn;
   // the step's maxima start over for the force pass to come (the step size
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(kBlock) k_gather(Params P, View src, View dst,
     dyn->Tv_max = 0.0f;
     dyn->nu_t_max = 0.0f;
     dyn->spacing_ratio = 1.0f;
+    if (P.heat_power == 0.0f) dyn->heat_inv_norm = 0.0f;  // no heater: no pass of this step sets it
   }
   const int na = dyn->n_alive;
   const int nch = num_chunks(na);
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(kBlock) k_gather(Params P, View src, View dst,
       const bool own = i >= own_lo && i < own_hi;
       if (is_fluid(ph) && own) cnt[0] = 1.0;
       else if (ph == kWall && own) cnt[1] = 1.0;
-      if (P.use_lists && is_fluid(ph)) dst.cell_fluid[cell_index(P, xyz(xp))] = 1;
+      if (P.use_lists && ph <= kWall) reinterpret_cast<uint8_t*>(dst.cell_kinds + cells[i])[ph] = 1;
     }
     publish_chunk<2>(R, c, cnt, sh);
   }
@@ -181,110 +184,206 @@ __global__ void __launch_bounds__(kBlock) k_gather(Params P, View src, View dst,
   }
 }
 
-// Neighbour lists of every particle in the reference's iteration order
-// (for_each_neighbor filtered by r^2 < support^2, self included), stored
-// transposed so a warp reads consecutive words.  mode LISTS_PHASE also fills
-// the ordered fluid / wall index lists from the gather's chunk offsets.
-__global__ void __launch_bounds__(kBlock, LIST_MIN_BLOCKS) k_build_lists(Params P, View V, Reduce R, int mode) {
+// Ordered index lists of the owned fluid and wall particles: for the chunk of
+// particle `first`, the entries of the particles the block itself handles
+// (kBlock / L of them, `first` on), from the gather's chunk offsets and the
+// particles' ranks inside the chunk.
+template <int L>
+__device__ inline void phase_lists(const Params& P, const View& V, const Reduce& R, int n, int first) {
   __shared__ int wcnt[2][kBlock / 32];
-  // each thread gathers a chunk of kNbrChunk entries here and stores it as
-  // one full 32-byte sector (column per thread: no bank conflicts)
-  __shared__ int stage[kNbrChunk][kBlock];
-#pragma unroll
-  for (int q = 0; q < kNbrChunk; ++q) stage[q][threadIdx.x] = 0;  // the unused tail of a last chunk
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = first / kChunk;
+  const int p = c * kChunk + threadIdx.x;
+  int own_lo, own_hi;
+  owned_layers(P, V.cell_begin, own_lo, own_hi);
+  const int ph = p < n ? ph_of(V.xp[p]) : kDead;
+  const bool own = p >= own_lo && p < own_hi;
+  const bool isf = own && is_fluid(ph), isw = own && ph == kWall;
+  const unsigned bf = __ballot_sync(0xffffffffu, isf), bw = __ballot_sync(0xffffffffu, isw);
+  if (lane == 0) {
+    wcnt[0][warp] = __popc(bf);
+    wcnt[1][warp] = __popc(bw);
+  }
+  __syncthreads();
+  if (p >= first && p < first + kBlock / L) {
+    int pf = 0, pw = 0;
+    for (int w = 0; w < warp; ++w) {
+      pf += wcnt[0][w];
+      pw += wcnt[1][w];
+    }
+    const unsigned lt = (1u << lane) - 1u;
+    if (isf) V.fluid_idx[(int)__ldcg(R.partials + c) + pf + __popc(bf & lt)] = p;
+    if (isw) V.wall_idx[(int)__ldcg(R.partials + R.max_chunks + c) + pw + __popc(bw & lt)] = p;
+  }
+  __syncthreads();
+}
+__device__ inline uint8_t near_bits(uint32_t kinds) {
+  return (uint8_t)((kinds & kCellLiquid ? kNearLiquid : 0) | (kinds & kCellVapor ? kNearVapor : 0) |
+                   (kinds & kCellWall ? kNearWall : 0));
+}
+// The candidates [s, e) of row of cells row9 (0-8, z-major) of the 27-cell
+// block, and the kinds of its cells added to `kinds`.  whole: every cell of
+// the row (positions that moved after the sort may have left their cell, and
+// lanes of one cell then walk the same ranges); otherwise the cells beyond
+// the support are dropped, as the cell scan does.  A wall keeps fluid
+// neighbours only, so a row of cells without fluid is empty for it.
+__device__ inline void list_row(const Params& P, const View& V, const CellWindow& W, int row9, bool whole, bool wall_i,
+                                int& s, int& e, uint32_t& kinds) {
+  s = e = 0;
+  const int z = W.cz + row9 / 3 - 1, y = W.cy + row9 % 3 - 1;
+  if (row9 >= 9 || z < W.z0 || z > W.z1 || y < W.y0 || y > W.y1) return;
+  int xs = W.x0, xe = W.x1;
+  if (!whole && !W.row(P, y, z, xs, xe)) return;
+  const int row = (z * P.ny + y) * P.nx;
+  uint32_t k = 0;
+  for (int x = xs; x <= xe; ++x) k |= __ldg(V.cell_kinds + row + x);
+  kinds |= k;
+  if (wall_i && !(k & (kCellLiquid | kCellVapor))) return;
+  s = __ldg(V.cell_begin + row + xs);
+  e = __ldg(V.cell_begin + row + xe + 1);
+}
+
+// Neighbour lists of every particle in the reference's iteration order
+// (for_each_neighbor filtered by r^2 < support^2, self included), with the
+// kinds of cells around each particle.  A wall's list holds its fluid
+// neighbours only: every pass that walks a wall's neighbours (the wall
+// boundary pass and its reverse) skips the other walls, so the fluid entries
+// in their order are all it needs.  mode LISTS_PHASE also fills the ordered
+// fluid / wall index lists.
+//
+// L = 1: a thread per particle, every lane on the same row at the same time.
+// An accepted candidate costs no branch: every candidate's index is stored at
+// the next place of the thread's ring of sixteen in shared memory (a column
+// per thread, no bank conflicts), and acceptance moves the place on.  After
+// every eight candidates the threads with a full chunk write it out as one
+// 32-byte sector.
+// L = LIST_LANES: the lanes share a particle (small tanks, where a thread's
+// walk over ~470 candidates sets the time): sixteen candidates per round,
+// four consecutive ones per lane, a prefix sum over the lanes for the places,
+// the list put together in shared memory and written in whole chunks.
+template <int L>
+__global__ void __launch_bounds__(kBlock, L == 1 ? 5 : 4) k_build_lists(Params P, View V, Reduce R, int mode) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kRing = 2 * kNbrChunk;
+  constexpr int kStride = kMaxNbr + 4;  // the pad takes what a longer list would add, and spreads the banks
+  constexpr int kPer = kBlock / L;  // particles per block
+  __shared__ __align__(16) int stage[L == 1 ? kRing * kPer : kPer * kStride];
   DynState* dyn = V.dyn;
   const int n = dyn->n;
-  const int nch = num_chunks(n);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   unsigned overflow = 0;
-  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
-    const int i = c * kChunk + threadIdx.x;
+  for (int first = blockIdx.x * kPer; first < n; first += gridDim.x * kPer) {
+    if (mode != LISTS_ONLY) phase_lists<L>(P, V, R, n, first);
+    const int i = first + threadIdx.x / L;
     const bool valid = i < n;
-    const float4 xpi = valid ? V.xp[i] : make_float4(0, 0, 0, 0);
-    const int ph = valid ? ph_of(xpi) : kDead;
-    if (mode != LISTS_ONLY) {
-      // ordered phase lists of the owned particles: chunk offset + rank inside the chunk
-      int own_lo, own_hi;
-      owned_layers(P, V.cell_begin, own_lo, own_hi);
-      const bool own = i >= own_lo && i < own_hi;
-      const bool isf = valid && own && is_fluid(ph), isw = valid && own && ph == kWall;
-      const unsigned bf = __ballot_sync(0xffffffffu, isf), bw = __ballot_sync(0xffffffffu, isw);
-      if (lane == 0) {
-        wcnt[0][warp] = __popc(bf);
-        wcnt[1][warp] = __popc(bw);
-      }
-      __syncthreads();
-      int pf = 0, pw = 0;
-      for (int w = 0; w < warp; ++w) {
-        pf += wcnt[0][w];
-        pw += wcnt[1][w];
-      }
-      const unsigned lt = (1u << lane) - 1u;
-      if (isf) V.fluid_idx[(int)__ldcg(R.partials + c) + pf + __popc(bf & lt)] = i;
-      if (isw) V.wall_idx[(int)__ldcg(R.partials + R.max_chunks + c) + pw + __popc(bw & lt)] = i;
-      __syncthreads();
-    }
-    if (!valid) continue;
+    const float4 xpi = V.xp[valid ? i : n - 1];
     const V3 xi = xyz(xpi);
+    const bool wall_i = ph_of(xpi) == kWall;
+    uint32_t kinds = 0;
     int cnt = 0;
-    const int t = threadIdx.x;
-    int4* chunk = reinterpret_cast<int4*>(V.nbr + (size_t)i * kNbrChunk);
-    const size_t cstride = (size_t)V.capacity * (kNbrChunk / 4);  // in int4
-    auto store_chunk = [&](int q) {
-      int4* dst = chunk + (size_t)q * cstride;
-      dst[0] = make_int4(stage[0][t], stage[1][t], stage[2][t], stage[3][t]);
-      dst[1] = make_int4(stage[4][t], stage[5][t], stage[6][t], stage[7][t]);
-    };
-    // A wall's list holds its fluid neighbours only: every pass that walks
-    // a wall's neighbours (the wall boundary pass and its reverse) skips the
-    // other walls, so the fluid entries in their order are all it needs;
-    // rows of cells with no fluid are not scanned.
-    const bool wall_i = ph == kWall;
-    const CellWindow W(P, xi);
-    for (int z = W.z0; z <= W.z1; ++z) {
-      for (int y = W.y0; y <= W.y1; ++y) {
-        // every row of the 27-cell block, whole: lanes in one cell then walk
-        // the same ranges (dropping rows beyond the support radius, as the
-        // cell scan does, saves candidates but splits the warp more)
-        const int xs = W.x0, xe = W.x1;
-        const int row = (z * P.ny + y) * P.nx;
-        if (wall_i) {
-          bool any = false;
-          for (int x = xs; x <= xe; ++x) any |= V.cell_fluid[row + x] != 0;
-          if (!any) continue;
-        }
-        const int s = __ldg(V.cell_begin + row + xs);
-        const int e = __ldg(V.cell_begin + row + xe + 1);
-        // candidates in groups of LIST_GROUP: all loads issued before the
-        // tests, so a thread has that many positions in flight
-        auto test = [&](const float4& xj, int j) {
-          const V3 rij = xi - xyz(xj);
-          const float r2 = norm2(rij);
-          if (r2 < P.support2 && (!wall_i || is_fluid(ph_of(xj)))) {
-            if (cnt < kMaxNbr) {
-              stage[cnt & (kNbrChunk - 1)][t] = j;
-              if ((cnt & (kNbrChunk - 1)) == kNbrChunk - 1) store_chunk(cnt / kNbrChunk);
+    if constexpr (L == 1) {
+      if (!valid) continue;
+      int* const column = stage + threadIdx.x;
+      auto flush = [&](int q) {  // chunk q out of its half of the ring
+        if (q >= kMaxNbr / kNbrChunk) return;
+        const int* h = column + (q & 1) * kNbrChunk * kPer;
+        int4* dst = reinterpret_cast<int4*>(V.nbr + ((size_t)q * V.capacity + i) * kNbrChunk);
+        dst[0] = make_int4(h[0], h[kPer], h[2 * kPer], h[3 * kPer]);
+        dst[1] = make_int4(h[4 * kPer], h[5 * kPer], h[6 * kPer], h[7 * kPer]);
+      };
+      int flushed = 0;  // chunks written
+      auto scan = [&](auto wall_c) {
+        constexpr bool kWallI = decltype(wall_c)::value;
+        const CellWindow W(P, xi);
+        for (int row9 = 0; row9 < 9; ++row9) {
+          int s, e;
+          list_row(P, V, W, row9, true, kWallI && wall_i, s, e, kinds);
+          for (int j = s; j < e; j += 8) {
+            // beyond the row's end: loaded (the array is padded), not accepted
+#pragma unroll
+            for (int h = 0; h < 8; h += 4) {
+              float4 x[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) x[u] = __ldg(V.xp + j + h + u);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                bool in = norm2(xi - xyz(x[u])) < P.support2 && j + h + u < e;
+                if (kWallI) in = in && (!wall_i || is_fluid(ph_of(x[u])));
+                column[(cnt & (kRing - 1)) * kPer] = j + h + u;
+                cnt += in ? 1 : 0;
+              }
             }
-            ++cnt;
+            if (cnt - flushed * kNbrChunk >= kNbrChunk) flush(flushed++);
           }
-        };
-        int j = s;
-        for (; j + LIST_GROUP <= e; j += LIST_GROUP) {
-          float4 xg[LIST_GROUP];
-#pragma unroll
-          for (int u = 0; u < LIST_GROUP; ++u) xg[u] = __ldg(V.xp + j + u);
-#pragma unroll
-          for (int u = 0; u < LIST_GROUP; ++u) test(xg[u], j + u);
         }
-        for (; j < e; ++j) test(__ldg(V.xp + j), j);
+      };
+      // a warp with a wall tests the phase for all its particles
+      if (__any_sync(__activemask(), wall_i)) scan(std::true_type{});
+      else scan(std::false_type{});
+      if (cnt > flushed * kNbrChunk) flush(flushed);  // the last, partial chunk
+    } else {
+      const int sub = lane & (L - 1), lead = lane & ~(L - 1);
+      int* const list = stage + (threadIdx.x / L) * kStride;
+      constexpr int kRowsPer = (9 + L - 1) / L;
+      int rs[kRowsPer], re[kRowsPer];  // rows sub, sub + L, ...: first and end candidate
+      {
+        const CellWindow W(P, xi);
+#pragma unroll
+        for (int q = 0; q < kRowsPer; ++q)
+          list_row(P, V, W, valid ? q * L + sub : 9, mode == LISTS_ONLY, wall_i, rs[q], re[q], kinds);
       }
+#pragma unroll
+      for (int row9 = 0; row9 < 9; ++row9) {
+        const int s = __shfl_sync(kAll, rs[row9 / L], lead + row9 % L);
+        const int e = __shfl_sync(kAll, re[row9 / L], lead + row9 % L);
+        for (int f = s; __any_sync(kAll, f < e); f += 4 * L) {
+          const int j = f + 4 * sub;
+          float4 x[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) x[u] = __ldg(V.xp + min(j + u, n - 1));
+          bool in[4];
+          int c = 0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            in[u] = j + u < e && norm2(xi - xyz(x[u])) < P.support2 && (!wall_i || is_fluid(ph_of(x[u])));
+            c += in[u];
+          }
+          int upto = c;  // accepted by the lanes up to this one
+#pragma unroll
+          for (int o = 1; o < L; o <<= 1) {
+            const int t = __shfl_up_sync(kAll, upto, o, L);
+            if (sub >= o) upto += t;
+          }
+          int k = min(cnt + upto - c, kMaxNbr);
+          cnt += __shfl_sync(kAll, upto, lead + L - 1);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (in[u]) list[k++] = j + u;
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < L; o <<= 1) kinds |= __shfl_xor_sync(kAll, kinds, o);
+      __syncwarp();
+      if (valid) {
+        const int chunks = (min(cnt, kMaxNbr) + kNbrChunk - 1) / kNbrChunk;
+        for (int q = sub; q < chunks; q += L) {
+          const int4* src = reinterpret_cast<const int4*>(list + q * kNbrChunk);
+          int4* dst = reinterpret_cast<int4*>(V.nbr + ((size_t)q * V.capacity + i) * kNbrChunk);
+          dst[0] = src[0];
+          dst[1] = src[1];
+        }
+      }
+      __syncwarp();  // the shared list is free again
+      if (!valid || sub != 0) continue;
     }
-    if (cnt < kMaxNbr && (cnt & (kNbrChunk - 1)) != 0) store_chunk(cnt / kNbrChunk);  // partial last chunk
     V.nbr_cnt[i] = cnt;
+    if (mode != LISTS_ONLY) V.near_kinds[i] = near_bits(kinds);
     if (cnt > kMaxNbr) overflow = CRYO_DEV_NBR_OVERFLOW;
   }
   if (overflow) atomicOr(&dyn->status, overflow);
 }
+template __global__ void k_build_lists<1>(Params, View, Reduce, int);
+template __global__ void k_build_lists<LIST_LANES>(Params, View, Reduce, int);
 
 // Neighbour list dump (test hook): counts, then the lists at given offsets.
 // stored = 0: the cell scan (every neighbour); 1: the lists of the last

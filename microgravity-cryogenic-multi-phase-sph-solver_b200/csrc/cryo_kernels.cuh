@@ -191,11 +191,12 @@ __device__ inline int num_chunks(int n) { return (n + kChunk - 1) / kChunk; }
 
 // grid (cryo_grid.cu)
 __global__ void k_keys(Params P, View V, CellSort S);
-__global__ void k_cell_scan(Params P, CellSort S, uint8_t* cell_fluid, unsigned* ticket);
+__global__ void k_cell_scan(Params P, CellSort S, uint32_t* cell_kinds, unsigned* ticket);
 __global__ void k_cell_scatter(Params P, CellSort S, DynState* dyn, int* cell_begin);
 __global__ void k_cell_order(Params P, CellSort S, const DynState* dyn, const int* cell_begin);
-__global__ void k_gather(Params P, View src, View dst, const uint32_t* perm, Reduce R, int reset_maxima);
+__global__ void k_gather(Params P, View src, View dst, const uint32_t* perm, const uint32_t* cells, Reduce R, int reset_maxima);
 enum { LISTS_ONLY = 0, LISTS_PHASE = 1 };
+template <int L>
 __global__ void k_build_lists(Params P, View V, Reduce R, int mode);
 __global__ void k_nbr_count(Params P, View V, int stored, int* counts);
 __global__ void k_nbr_fill(Params P, View V, int stored, const long long* offsets, int* list);
@@ -218,7 +219,7 @@ enum { FORCE_TRANSPORT = 1, FORCE_MOMENTUM = 2, FORCE_CSF = 4, FORCE_AKINCI = 8,
   __global__ void k_eos(Params P, View V);                                          \
   __global__ void k_wall(Params P, View V);                                         \
   template <int TAPE>                                                               \
-  __global__ void k_interface(Params P, View V, Reduce R, int heat_sum);            \
+  __global__ void k_interface(Params P, View V);                                    \
   __global__ void k_sps(Params P, View V);                                          \
   __global__ void k_smooth_normals(Params P, View V);                               \
   template <int WHAT>                                                               \
@@ -233,8 +234,8 @@ CRYO_FIELD_KERNELS
 namespace fast {
 CRYO_FIELD_KERNELS
 }
-// heat_sum of k_interface: 0 none, 1 when thermal is on (step), 2 always (operator call)
 // TAPE: also store the sums into V.tape (the recomputation of a differentiated window).
+constexpr int INTERFACE_BLOCK = 128;
 constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
 // Block shape of the force pass.  The pass is bound by the latency of each
 // particle's neighbour chain, so what matters is how many particles are in
@@ -257,21 +258,19 @@ constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
 constexpr int forces_min_blocks(int what) {
   return (what >= 0 && (what & (FORCE_CSF | FORCE_THERMAL))) ? FORCES_MIN_BLOCKS_HEAVY : FORCES_MIN_BLOCKS;
 }
-// Neighbour-list build: candidate positions loaded per group, and the block
-// count per SM the register cap keeps resident.
 // Neighbour-loop unroll of the force-pass variants with surface tension or
 // heat (the two-phase tanks): 2 takes the 4 M-particle LH2 sphere 3 % faster,
 // no spills.
 #ifndef FORCES_UNROLL_HEAVY
 #define FORCES_UNROLL_HEAVY 2
 #endif
-#ifndef LIST_GROUP
-#define LIST_GROUP 4
+// Neighbour-list build: LIST_LANES lanes per particle up to LIST_LANES_MAX
+// particles, one above (k_build_lists).
+constexpr int LIST_LANES = 4;
+constexpr int kListPad = 8;  // records the build may load beyond the last particle
+#ifndef LIST_LANES_MAX
+#define LIST_LANES_MAX 300000
 #endif
-#ifndef LIST_MIN_BLOCKS
-#define LIST_MIN_BLOCKS 4
-#endif
-
 // integrator + phase change (cryo_phase.cu)
 __global__ void k_kick_drift(Params P, View V, int continuity, int tvf);
 enum { KICK_SOURCES = 1, KICK_HEAT = 2 };
@@ -289,6 +288,7 @@ __global__ void k_scale_velocities(View V, float factor, int scale_vmax);
 enum { BEGIN_STEP = 0, BEGIN_RATES = 1 };
 __global__ void k_begin_step(Params P, View V, int mode);
 __global__ void k_heat_norm(Params P, View V, Reduce R);
+__global__ void k_heat_sum(Params P, View V, Reduce R);
 // The ullage pressure and saturation temperature from the phase sums
 // (sph_solver.cu:586-607).
 __device__ inline void saturation_update(const Params& P, DynState* d, bool closed, double m_liq, double m_vap,

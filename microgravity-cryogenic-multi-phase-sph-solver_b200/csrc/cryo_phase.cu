@@ -18,8 +18,10 @@ __global__ void __launch_bounds__(kBlock) k_kick_drift(Params P, View V, int con
   }
 }
 
-// phase_change_sources (phase_change.cu:77-137) for particle i.
-__device__ inline void pc_source_one(const Params& P, const View& V, int i, float T_sat, float dt, float4 xp) {
+// phase_change_sources (phase_change.cu:77-137) for particle i.  mark: sources
+// are noted in the cells around them (View::cell_kinds).
+__device__ inline void pc_source_one(const Params& P, const View& V, int i, float T_sat, float dt, float4 xp,
+                                     bool mark) {
   const int ph = ph_of(xp);
   int fl = fl_of(xp) & ~kScratchMask;
   float out_m = 0.0f, out_h = 0.0f;
@@ -66,6 +68,18 @@ __device__ inline void pc_source_one(const Params& P, const View& V, int i, floa
   }
   V.pc[i] = make_float4(out_m, out_h, 0.0f, V.pc[i].w);
   reinterpret_cast<float*>(V.xp + i)[3] = pack_pf(ph, fl);
+  if (mark && (fl & kSource)) {
+    // the cells whose particles can have this source among their neighbours
+    // (the cell it was sorted into: it has not moved since); one lane per cell
+    int cx, cy, cz;
+    cell_coords(P, xyz(xp), cx, cy, cz);
+    const unsigned peers = __match_any_sync(__activemask(), (cz * P.ny + cy) * P.nx + cx);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1)
+      for (int z = max(cz - 1, 0); z <= min(cz + 1, P.nz - 1); ++z)
+        for (int y = max(cy - 1, 0); y <= min(cy + 1, P.ny - 1); ++y)
+          for (int x = max(cx - 1, 0); x <= min(cx + 1, P.nx - 1); ++x)
+            reinterpret_cast<uint8_t*>(V.cell_kinds + (z * P.ny + y) * P.nx + x)[3] = 1;
+  }
 }
 
 // kick (sph_solver.cu:36-46).  flags & KICK_SOURCES: the phase-change sources
@@ -91,7 +105,7 @@ __global__ void __launch_bounds__(kBlock) k_kick(Params P, View V, int flags) {
       if (thermal) T += a4.w * dt;
       V.vT[i] = f4(v, T);
     }
-    if (do_src) pc_source_one(P, V, i, T_sat, dt, xp);
+    if (do_src) pc_source_one(P, V, i, T_sat, dt, xp, P.use_lists && !P.slab);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && (flags & KICK_HEAT)) {
     if (thermal && dyn->heat_inv_norm > 0.0f) dyn->heat_input += (double)P.heat_power * (double)dt;
@@ -101,7 +115,7 @@ __global__ void __launch_bounds__(kBlock) k_kick(Params P, View V, int flags) {
 __global__ void __launch_bounds__(kBlock) k_pc_sources(Params P, View V) {
   const DynState* dyn = V.dyn;
   const int n = dyn->n;
-  PARTICLE_LOOP(i, n) pc_source_one(P, V, i, dyn->T_sat, dyn->dt, V.xp[i]);
+  PARTICLE_LOOP(i, n) pc_source_one(P, V, i, dyn->T_sat, dyn->dt, V.xp[i], false);
 }
 
 // phase_change_normalize (phase_change.cu:139-172); with `sums` (step mode)
@@ -180,7 +194,11 @@ __global__ void __launch_bounds__(kBlock) k_pc_apply(Params P, View V, int gated
     const float mi = mr.x;
     const float Vi = mi / mr.y;
     float in_m = 0.0f, in_H = 0.0f;
-    if (!(fl & kDying)) {
+    // in a step, a particle with no source in the cells around it receives
+    // nothing (a slab's ghosts are flagged by their owners: no marks there)
+    const bool receives = !(fl & kDying) && (!gated || !P.use_lists || P.slab ||
+                                             (V.cell_kinds[cell_index(P, xyz(xpi))] & kCellNearSource));
+    if (receives) {
       for_each_nbr(P, V, i, xyz(xpi), [&](int j, float4 xj, V3, float r2) {
         // only flagged sources carry out_m > 0 (pc_source_one), so the
         // others are passed over without reading their pc record

@@ -151,25 +151,35 @@ __global__ void __launch_bounds__(kBlock) k_wall(Params P, View V) {
   }
 }
 
-// compute_interface_fields (surface_tension.cu:5-85).  With heat_sum the FP64
-// sum of heat_w over fluid particles (sph_solver.cu:101-104) is reduced in the
-// same pass and heat_inv_norm is set (sph_solver.cu:466-472); the CSF unit
-// normal (smooth_interface_normals without smoothing, surface_tension.cu:91-101)
-// is written when the CSF model is active.
+// compute_interface_fields (surface_tension.cu:5-85); the CSF unit normal
+// (smooth_interface_normals without smoothing, surface_tension.cu:91-101) is
+// written when the CSF model is active.  The heat weights it leaves are summed
+// by k_heat_sum, where there is a heater.  Particles by walls and interfaces
+// walk their lists and the others do not, so the blocks are small, none waits
+// for its other warps, and there is one per INTERFACE_BLOCK particles: the
+// warps that finish at once make room for others.
 template <int TAPE>
-__global__ void __launch_bounds__(kBlock) k_interface(Params P, View V, Reduce R, int heat_sum) {
-  __shared__ double sh[kBlock / 32];
+__global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V) {
   const Range rg = fluid_range(P, V);
-  const int nch = num_chunks(rg.count);
   const bool write_ns = P.csf_active && !P.csf_smooth;
-  const int own_lo = V.dyn->own_lo, own_hi = V.dyn->own_hi, n_sorted = V.dyn->n_sorted;
-  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
-    const int t = c * kChunk + threadIdx.x;
-    double hsum[1] = {0.0};
-    if (t < rg.count) {
+  {
+    PARTICLE_LOOP(t, rg.count) {
       const int i = particle_at(rg, t);
       const float4 xpi = V.xp[i];
       const int ph = ph_of(xpi);
+      // A particle with no wall and none of the other phase in the cells
+      // around it: s_other is 0, so alpha is 0 whatever s_all is, and every
+      // other sum stays empty.  Away from walls and interfaces (four fifths of
+      // a 4 M-particle sphere) the pass then walks no list.
+      if (!TAPE && P.use_lists && P.st_model != CRYO_ST_AKINCI && is_fluid(ph) &&
+          !(V.near_kinds[i] & (kNearWall | (ph == kVapor ? kNearLiquid : kNearVapor)))) {
+        V.wall_w[i] = 0.0f;
+        V.heat_w[i] = 0.0f;
+        V.vwp[i] = make_float4(0.0f, 0.0f, 0.0f, V.vwp[i].w);
+        V.nrm[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (write_ns) V.ns4[i] = make_float4(0.0f, 0.0f, 0.0f, V.ns4[i].w);
+        continue;
+      }
       if (is_fluid(ph)) {
         const V3 xi = xyz(xpi);
         const float ci = ph == kLiquid ? 1.0f : 0.0f;
@@ -224,7 +234,6 @@ __global__ void __launch_bounds__(kBlock) k_interface(Params P, View V, Reduce R
         const float alpha = s_all > 0.0f ? s_other / s_all : 0.0f;
         V.wall_w[i] = ww;
         V.heat_w[i] = hw;
-        if (owned(own_lo, own_hi, n_sorted, i)) hsum[0] = (double)hw;
         if (P.st_model == CRYO_ST_AKINCI) {
           V.nrm[i] = f4(ph == kLiquid ? akn * (-P.h) : V3{0, 0, 0}, alpha);
         } else {
@@ -265,26 +274,11 @@ __global__ void __launch_bounds__(kBlock) k_interface(Params P, View V, Reduce R
         }
       }
     }
-    if (heat_sum) publish_chunk<1>(R, c, hsum, sh);
-  }
-  if (heat_sum && last_block(R.ticket)) {
-    DynState* dyn = V.dyn;
-    const double S = block_sum_partials(R, 0, nch);
-    if (threadIdx.x != 0) return;
-    dyn->heat_sum = S;
-    if (P.slab) return;  // the slabs set heat_inv_norm from their combined sums
-    if (heat_sum == 2 || dyn->thermal_on) {
-      if (P.heat_power != 0.0f) {
-        dyn->heat_inv_norm = S > 0 ? (float)(1.0 / S) : 0.0f;
-      } else {
-        dyn->heat_inv_norm = 0.0f;
-      }
-    }
   }
 }
 
-template __global__ void k_interface<0>(Params, View, Reduce, int);
-template __global__ void k_interface<1>(Params, View, Reduce, int);
+template __global__ void k_interface<0>(Params, View);
+template __global__ void k_interface<1>(Params, View);
 
 // compute_sps_viscosity (navier_stokes.cu:71-119)
 __global__ void __launch_bounds__(kBlock) k_sps(Params P, View V) {

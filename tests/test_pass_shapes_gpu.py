@@ -1,7 +1,9 @@
-"""The cell sort at the sizes where a remainder can go wrong, bit for bit."""
+"""The cell sort and the neighbour-list build at the sizes where a change of
+launch shape or a remainder can go wrong, bit for bit."""
 import numpy as np
 import pytest
 
+import CryoSPH as cs
 import cryo_cabi as cabi
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +48,42 @@ def test_cell_sort_is_the_stable_sort(cuda_device, n, dense, outside):
         assert np.array_equal(perm, order) and np.array_equal(keys, key[order])
         count = np.bincount(key, minlength=info["num_cells"])
         assert np.array_equal(end - begin, count)
+
+
+def assert_stored_equal_scan(g, phase):
+    sc, sl = g.neighbor_lists(stored=True)
+    gc, gl = g.neighbor_lists()
+    owner = np.repeat(np.arange(len(gc)), gc)
+    keep = (phase[owner] != 2) | (phase[gl] <= 1)  # a wall's stored list holds its fluid neighbours
+    assert np.array_equal(sc, np.bincount(owner[keep], minlength=len(gc)))
+    assert np.array_equal(sl, gl[keep])
+
+
+@pytest.mark.parametrize("n", [1, 3, 7, 9, 63, 64, 65, 255, 1025, 4099])
+def test_lists_of_random_clouds(cuda_device, n):
+    g = cabi.Context(free_surface_config(0.012), cabi.py_fluid(cabi.FLUID_H2O))
+    p = cloud(n, 7 * n)
+    p["phase"][::5] = 2  # some walls among them
+    g.set_particles(p, LO, HI)
+    g.run_pass("grid_build")
+    assert_stored_equal_scan(g, g.field("phase"))
+
+
+def big_tank():
+    water = cs.FluidProperties.water()
+    fill = cs.FillSpec()
+    fill.fill_fraction = 0.55
+    return water, cs.tank_particles(cs.BoxTank(0.27, 0.25, 0.26), water, 0.004, fill), cs.tank_domain(
+        cs.BoxTank(0.27, 0.25, 0.26), 0.004, 3)
+
+
+def test_lists_of_a_large_tank(cuda_device):
+    """More particles than the list build shares lanes over, in the one-thread shape."""
+    _, p, (lo, hi) = big_tank()
+    n = len(p["mass"])
+    assert n > 300_000
+    g = cabi.Context(cabi.py_config(dx=0.004, thermo_mode=1), cabi.py_fluid(cabi.FLUID_H2O))
+    g.set_particles({"x": p["position"], "m": p["mass"], "rho": p["density"], "T": p["temperature"],
+                     "phase": p["phase"], "nrm": p["normal"]}, lo, hi)
+    g.run_pass("grid_build")
+    assert_stored_equal_scan(g, g.field("phase"))
