@@ -215,7 +215,7 @@ void cryo_ctx::sort_and_gather(int src, int list_mode, bool reset_maxima) {
 }
 
 void cryo_ctx::build_lists(const View& V, int mode) {
-  if (loaded_n <= LIST_LANES_MAX)
+  if (crowded(loaded_n) <= LIST_LANES_MAX)
     LAUNCH(k_build_lists<LIST_LANES>, list_blocks(LIST_LANES), kBlock, P, V, reduce(), mode);
   else
     LAUNCH(k_build_lists<1>, list_blocks(1), kBlock, P, V, reduce(), mode);
@@ -228,13 +228,20 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
   const View V = view(s);
   if (maxima_reset) LAUNCH(k_begin_step, 1, 1, P, V, BEGIN_RATES);
   if (!density_done) {
-    FIELD_LAUNCH(k_density, G, kBlock, P, V, 1);
+    if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
+    else FIELD_LAUNCH(k_density, G, kBlock, P, V, 1);
     slab_point(SLAB_HALO, s);
   }
-  FIELD_LAUNCH(k_wall, G, kBlock, P, V);
+  if (rate_lanes(loaded_n - loaded_fluid, WALL_LANES_MAX)) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
+  else FIELD_LAUNCH(k_wall, G, kBlock, P, V);
   slab_point(SLAB_HALO, s);
-  if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V);
-  else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V);
+  if (rate_lanes(loaded_fluid, INTERFACE_LANES_MAX)) {
+    if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V);
+    else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V);
+  } else {
+    if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V);
+    else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V);
+  }
   // without a heater there is nothing to normalise: the force pass reads a zero power
   if (P.thermal && P.heat_power != 0.0f) LAUNCH(k_heat_sum, G, kBlock, P, V, reduce());
   slab_point(P.thermal ? SLAB_HEAT : SLAB_HALO, s);
@@ -247,28 +254,31 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
     slab_point(SLAB_HALO, s);
   }
   const int GF = forces_blocks();
+  const bool laned = rate_lanes(loaded_fluid, FORCES_LANES_MAX);
+  const int GL = lane_blocks(FORCES_LANED_BLOCK);
   int what = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
   if (P.csf_active) what |= FORCE_CSF;
   if (P.st_model == CRYO_ST_AKINCI) what |= FORCE_AKINCI;
   if (P.density_mode == CRYO_DENSITY_CONTINUITY) what |= FORCE_DRHO;
   if (P.thermal) what |= FORCE_THERMAL;
-  if (tape) {  // the recomputation of a differentiated window: variants that also store their sums
-    switch (what) {
-      case FORCE_BASE: FIELD_LAUNCH(k_forces_t<FORCE_BASE | FORCE_TAPE>, GF, FORCES_BLOCK, P, V, what); break;
-      case FORCE_BASE | FORCE_THERMAL:
-        FIELD_LAUNCH(k_forces_t<FORCE_BASE | FORCE_THERMAL | FORCE_TAPE>, GF, FORCES_BLOCK, P, V, what);
-        break;
-      case FORCE_BASE | FORCE_CSF: FIELD_LAUNCH(k_forces_t<FORCE_BASE | FORCE_CSF | FORCE_TAPE>, GF, FORCES_BLOCK, P, V, what); break;
-      case FORCE_BASE | FORCE_CSF | FORCE_THERMAL:
-        FIELD_LAUNCH(k_forces_t<FORCE_BASE | FORCE_CSF | FORCE_THERMAL | FORCE_TAPE>, GF, FORCES_BLOCK, P, V, what);
-        break;
+  // (a pass of a differentiated window's recomputation also stores its sums;
+  // such a window is in the exact arithmetic)
+#define FORCES_CASE(W)                                                       \
+  case W:                                                                    \
+    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);   \
+    else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);             \
+    break;
+  if (tape) {
+    switch (what | FORCE_TAPE) {
+      FORCES_CASE(FORCE_BASE | FORCE_TAPE)
+      FORCES_CASE(FORCE_BASE | FORCE_THERMAL | FORCE_TAPE)
+      FORCES_CASE(FORCE_BASE | FORCE_CSF | FORCE_TAPE)
+      FORCES_CASE(FORCE_BASE | FORCE_CSF | FORCE_THERMAL | FORCE_TAPE)
       default: throw std::runtime_error("internal: no taped force pass for this configuration");
     }
     return;
   }
   switch (what) {
-#define FORCES_CASE(W) \
-  case W: FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W); break;
     FORCES_CASE(FORCE_BASE)
     FORCES_CASE(FORCE_BASE | FORCE_THERMAL)
     FORCES_CASE(FORCE_BASE | FORCE_DRHO)
@@ -337,15 +347,15 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
-    LAUNCH(k_pc_normalize, G, kBlock, P, V, R, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, k_pc_normalize, P, V, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.pc, tape->pc2, nullptr, nullptr, dyn);
-    LAUNCH(k_pc_apply, G, kBlock, P, V, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, k_pc_apply, P, V, R, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT2, tape->m2, V.mrps, dyn);
     const bool reb = P.vapor_rebalance > 0.0f && has_vapor;
     if (reb) {
-      LAUNCH(k_rebalance1, G, kBlock, P, V, 1);
+      PASS_LAUNCH(crowded(loaded_fluid) <= PASS_LANES_MAX, k_rebalance1, P, V, 1);
       slab_point(SLAB_HALO, d);
     }
     LAUNCH(k_rebalance2_mark, G, kBlock, P, V, R, split_flag, reb ? 1 : 0, 1);
@@ -640,7 +650,7 @@ uintptr_t cryo_stream(const cryo_ctx* ctx) { return reinterpret_cast<uintptr_t>(
 // ParticleSystem::upload, particle_system.cpp:73-93): checks, parameters,
 // capacity and grid for n particles, then (finish_load) the clean scratch and
 // the reset scalar block once the particles are in set[0].
-void cryo_ctx::begin_load(int n, bool vap, const float* lo, const float* hi) {
+void cryo_ctx::begin_load(int n, int n_fluid, bool vap, const float* lo, const float* hi) {
   if (vap && cfg.surface_tension == CRYO_ST_AKINCI)
     throw std::invalid_argument(
         "Solver: the Akinci surface-tension model is a free-surface (liquid-only) model; use CSF when vapour "
@@ -675,10 +685,11 @@ void cryo_ctx::begin_load(int n, bool vap, const float* lo, const float* hi) {
   // optimisation or restart loop) keeps the captured step graphs: every
   // argument they hold is unchanged, so its first step replays instead of
   // capturing again.  Anything else drops them.
-  const bool same = n == old_n && old_arena == arena.base && old_cells == cell_begin &&
+  const bool same = n == old_n && n_fluid == loaded_fluid && old_arena == arena.base && old_cells == cell_begin &&
                     std::memcmp(&old_P, &P, sizeof(Params)) == 0;
   if (!same) this->invalidate_graphs();
   loaded_n = n;
+  loaded_fluid = n_fluid;
   cur = 0;
 }
 
@@ -921,7 +932,7 @@ int cryo_build_tank(cryo_ctx* c, const cryo_geom_node_t* nodes, int n_nodes, con
         lo[q] = blo[q] - pad;
         hi[q] = bhi[q] + pad;
       }
-      c->begin_load(n, vapor, lo, hi);
+      c->begin_load(n, kept, vapor, lo, hi);
       const View V = c->view(0);
       const int gw = std::max(1, std::min((int)((nw + kBlock - 1) / kBlock), c->sm_count * 8));
       if (nw > 0) {
@@ -1501,10 +1512,10 @@ int cryo_pass(cryo_ctx* c, int pass) {
         if (P.use_lists) c->build_lists(V, LISTS_ONLY);
         break;
       case CRYO_PASS_PC_SOURCES: k_pc_sources<<<G, kBlock, 0, st>>>(P, V); break;
-      case CRYO_PASS_PC_NORMALIZE: k_pc_normalize<<<G, kBlock, 0, st>>>(P, V, R, 0); break;
-      case CRYO_PASS_PC_APPLY: k_pc_apply<<<G, kBlock, 0, st>>>(P, V, 0); break;
+      case CRYO_PASS_PC_NORMALIZE: k_pc_normalize<1><<<G, kBlock, 0, st>>>(P, V, 0); break;
+      case CRYO_PASS_PC_APPLY: k_pc_apply<1><<<G, kBlock, 0, st>>>(P, V, R, 0); break;
       case CRYO_PASS_REBALANCE:
-        k_rebalance1<<<G, kBlock, 0, st>>>(P, V, 0);
+        k_rebalance1<1><<<G, kBlock, 0, st>>>(P, V, 0);
         LAUNCH_CHECK();
         k_rebalance2_mark<<<G, kBlock, 0, st>>>(P, V, R, c->split_flag, 1, 0);
         break;

@@ -561,6 +561,78 @@ __device__ inline void for_each_nbr_pf(const Params& P, const View& V, int i, V3
   }
 }
 
+// The neighbours of particle i handed out L at a time to the L lanes that
+// share the particle, in the order for_each_nbr visits them: take() gives each
+// lane its neighbour of the round (-1: none).  With a list, the next round's
+// indices and positions are in flight while the current one is processed;
+// without one (lists off, or more neighbours than it holds) the lanes search
+// the cells, L candidates a round, and a candidate beyond the support is none.
+// more() is the same in all lanes of a particle; a warp keeps taking rounds
+// until no particle of its lanes has any left.
+template <int L>
+struct NbrRounds {
+  const Params& P;
+  const View& V;
+  const int i, sub;
+  const V3 xi;
+  bool list;
+  int k = 0, c = 0;           // list: entries handed out, entries
+  int jn = -1, jnn = -1;      // list: this lane's index of the next round and of the one after
+  float4 xn;                  // list: the position of jn
+  int row9 = 9, j0 = 0, e = 0;  // search: row of cells, its next candidate and end
+  __device__ NbrRounds(const Params& P_, const View& V_, int i_, V3 xi_, int sub_, bool live)
+      : P(P_), V(V_), i(i_), sub(sub_), xi(xi_), xn(make_float4(0, 0, 0, 0)) {
+    const int n = !live ? 0 : (P.use_lists ? __ldg(V.nbr_cnt + i) : kMaxNbr + 1);
+    list = n <= kMaxNbr;
+    if (list) {
+      c = n;
+      jn = entry(sub);
+      if (jn >= 0) xn = __ldg(V.xp + jn);
+      jnn = entry(L + sub);
+    } else {
+      row9 = -1;
+      next_row();
+    }
+  }
+  __device__ int entry(int q) const {
+    return q < c ? __ldg(V.nbr + ((size_t)(q / kNbrChunk) * V.capacity + i) * kNbrChunk + q % kNbrChunk) : -1;
+  }
+  __device__ void next_row() {
+    const CellWindow W(P, xi);
+    j0 = e = 0;
+    while (++row9 < 9) {
+      const int z = W.cz + row9 / 3 - 1, y = W.cy + row9 % 3 - 1;
+      int xs, xe;
+      if (z < W.z0 || z > W.z1 || y < W.y0 || y > W.y1 || !W.row(P, y, z, xs, xe)) continue;
+      const int row = (z * P.ny + y) * P.nx;
+      j0 = __ldg(V.cell_begin + row + xs);
+      e = __ldg(V.cell_begin + row + xe + 1);
+      if (j0 < e) return;
+    }
+  }
+  __device__ bool more() const { return list ? k < c : row9 < 9; }
+  __device__ int take(float4& xj) {
+    int j = -1;
+    if (list) {
+      j = jn;
+      xj = xn;
+      k += L;
+      jn = jnn;
+      if (jn >= 0) xn = __ldg(V.xp + jn);
+      jnn = entry(k + L + sub);
+    } else {
+      if (j0 + sub < e) {
+        j = j0 + sub;
+        xj = __ldg(V.xp + j);
+        if (!(norm2(xi - xyz(xj)) < P.support2)) j = -1;
+      }
+      j0 += L;
+      if (j0 >= e && row9 < 9) next_row();
+    }
+    return j;
+  }
+};
+
 // The particles a pass visits: with lists, an ordered phase index list
 // (fluid or wall); otherwise every particle (the pass filters by phase).
 struct Range {

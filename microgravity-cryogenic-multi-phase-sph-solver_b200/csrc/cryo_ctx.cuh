@@ -51,6 +51,15 @@ struct CudaError : std::runtime_error {
     this->after_launch();                        \
   } while (0)
 
+// A phase-change pass in the shape its size asks for.
+#define PASS_LAUNCH(SMALL, K, ...)                                  \
+  do {                                                              \
+    if (SMALL)                                                      \
+      LAUNCH(K<PASS_LANES>, lane_blocks(), kBlock, __VA_ARGS__);    \
+    else                                                            \
+      LAUNCH(K<1>, grid_blocks(), kBlock, __VA_ARGS__);             \
+  } while (0)
+
 // A kernel of cryo_physics.cu in the context's field arithmetic (exact: the
 // reference's IEEE sequence; fast: contracted, see cryo_kernels.cuh).
 #define FIELD_KERNEL(ctx, K) ((ctx)->fast_fields ? &fast::K : &exact::K)
@@ -198,6 +207,7 @@ struct cryo_ctx {
   bool has_particles = false, initialized = false, has_vapor = false;
   bool lists_built = false;  // the neighbour lists of the current particles exist
   int loaded_n = -1;  // particle count of the last set_particles / build_tank
+  int loaded_fluid = 0;  // the liquid and vapour particles among them
   float char_length = 0;
   float pass_dt = 0;
 
@@ -401,6 +411,18 @@ struct cryo_ctx {
     const int need = (span() + per_block - 1) / per_block;
     return std::max(1, std::min(need, sm_count * 8));
   }
+  // Which shape a neighbour pass takes depends on the particles loaded, in an
+  // ensemble on those that step side by side: lanes pay only while they would
+  // otherwise be idle.  Both shapes give the same bits, so a tank steps alike
+  // alone and in an ensemble.  The rate passes have lanes in the exact
+  // arithmetic only (cryo_lanes.cu), the phase-change passes always.
+  int crowd = 0;  // while an ensemble captures: the particles of the tanks side by side
+  int crowded(int own) const { return std::max(own, crowd); }
+  bool rate_lanes(int count, int most) const { return !fast_fields && P.use_lists && crowded(count) <= most; }
+  int lane_blocks(int block = kBlock) const {
+    const int per_block = block / PASS_LANES * grid_tile;
+    return std::max(1, std::min((span() + per_block - 1) / per_block, sm_count * 64));
+  }
   int interface_blocks() const {
     const int per_block = INTERFACE_BLOCK * grid_tile;
     return std::max(1, (span() + per_block - 1) / per_block);
@@ -519,7 +541,7 @@ struct cryo_ctx {
   // --------------------------------------------------- parameter lowering
   void init_params();
   void configure_grid(const float* lo, const float* hi);
-  void begin_load(int n, bool vapor, const float* lo, const float* hi);
+  void begin_load(int n, int n_fluid, bool vapor, const float* lo, const float* hi);
   void finish_load(int n, uint32_t next_id);
 
   // ------------------------------------------------------ step pieces

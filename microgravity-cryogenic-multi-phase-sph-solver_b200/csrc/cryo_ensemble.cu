@@ -89,6 +89,11 @@ struct cryo_ensemble {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int launches = 0;
+    // fluid particles of the tanks that step side by side: the branches' share
+    long long fluid = 0;
+    for (const cryo_ctx* c : tanks) fluid += c->loaded_fluid;
+    const int crowd =
+        (int)std::min<long long>(fluid * branches() / std::max<long long>((long long)tanks.size(), 1), 1 << 30);
     try {
       CK(cudaEventRecord(fork, stream));
       for (const auto& br : branches_plan) {
@@ -100,9 +105,13 @@ struct cryo_ensemble {
           struct TileScope {
             cryo_ctx* c;
             int saved;
-            ~TileScope() { c->grid_tile = saved; }
+            ~TileScope() {
+              c->grid_tile = saved;
+              c->crowd = 0;
+            }
           } scope{c, c->grid_tile};
           c->grid_tile = tile;
+          c->crowd = crowd;
           for (int k = 0; k < steps; ++k) {
             const long long c0 = c->launch_counter;
             c->enqueue_step((built_cur[t] + q + k) & 1);

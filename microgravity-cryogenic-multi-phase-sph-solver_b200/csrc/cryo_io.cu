@@ -250,13 +250,17 @@ int cryo_set_particles_columns(cryo_ctx* c, const cryo_host_columns_t* p, const 
     if (!p->x || !p->m || !p->rho || !p->T || !p->phase)
       throw std::invalid_argument("Solver::set_particles: x, m, rho, T and phase are required");
     bool vap = false;
-    for (int i = 0; i < n; ++i) vap |= p->phase[i] == CRYO_VAPOR;
+    int fluid = 0;
+    for (int i = 0; i < n; ++i) {
+      vap |= p->phase[i] == CRYO_VAPOR;
+      fluid += is_fluid(p->phase[i]);
+    }
     uint32_t next_id = (uint32_t)n;
     if (p->id) {
       next_id = 0;
       for (int i = 0; i < n; ++i) next_id = std::max(next_id, p->id[i] + 1);
     }
-    c->begin_load(n, vap, lo, hi);
+    c->begin_load(n, fluid, vap, lo, hi);
     const IoLayout L = io_layout((size_t)n);
     c->io_reserve(L.bytes);
     char* h = c->io_host;

@@ -187,6 +187,19 @@ __device__ inline void publish_chunk(const Reduce& R, int c, double (&v)[NV], do
     }
   __syncthreads();  // sh is free again
 }
+// Sums over neighbours that L lanes visit side by side (NbrRounds): every lane
+// brings its neighbour's terms t, and each sum takes the lanes' terms one
+// after another in lane order -- the neighbours' order -- so that every lane
+// holds the sums a single thread walking the list would have.  Every lane of
+// the warp must take part.
+template <int L, int K>
+__device__ inline void add_terms(float (&s)[K], const float (&t)[K]) {
+  const int lead = L > 1 ? (threadIdx.x & 31) & ~(L - 1) : 0;
+#pragma unroll
+  for (int u = 0; u < L; ++u)
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k] += L > 1 ? __shfl_sync(0xffffffffu, t[k], lead + u) : t[k];
+}
 __device__ inline int num_chunks(int n) { return (n + kChunk - 1) / kChunk; }
 
 // grid (cryo_grid.cu)
@@ -234,6 +247,15 @@ CRYO_FIELD_KERNELS
 namespace fast {
 CRYO_FIELD_KERNELS
 }
+// cryo_lanes.cu: the exact passes with PASS_LANES lanes per particle.
+namespace lanes {
+__global__ void k_density(Params P, View V);
+__global__ void k_wall(Params P, View V);
+template <int TAPE>
+__global__ void k_interface(Params P, View V);
+template <int WHAT>
+__global__ void k_forces_t(Params P, View V);
+}
 // TAPE: also store the sums into V.tape (the recomputation of a differentiated window).
 constexpr int INTERFACE_BLOCK = 128;
 constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
@@ -271,13 +293,46 @@ constexpr int kListPad = 8;  // records the build may load beyond the last parti
 #ifndef LIST_LANES_MAX
 #define LIST_LANES_MAX 300000
 #endif
+// The neighbour passes that come in two shapes, one thread per particle and
+// PASS_LANES lanes per particle, take the second up to these counts (fluid
+// particles; walls for the wall pass; in an ensemble those of the tanks that
+// step side by side).  Lanes shorten the chain of a particle's ~75 neighbours
+// but add shuffles and rows, so they pay while the chip has room for the
+// threads.  Measured one thread against lanes, us per launch (event overhead
+// of ~5 us included):
+//   fluid particles        1 000      14 500     61 000     82 350
+//   force pass, exact    158 / 36   159 / 58       -       153 / 190
+//   density               29 / 15    32 / 19    31 / 45    35 / 52
+//   interface             77 / 22    78 / 28    68 / 42    62 / 44
+//   phase-change apply    31 / 18    39 / 21    44 / 30
+//   vapour rebalance      33 / 17    36 / 21    37 / 39
+// and the wall pass 21 / 15 at 12 000 walls, 23 / 15 at 30 000, 23 / 27 at
+// 121 000.
+constexpr int PASS_LANES = 8;
+constexpr int FORCES_LANED_BLOCK = 128;
+#ifndef FORCES_LANES_MAX
+#define FORCES_LANES_MAX 45000
+#endif
+#ifndef PASS_LANES_MAX
+#define PASS_LANES_MAX 40000
+#endif
+#ifndef INTERFACE_LANES_MAX
+#define INTERFACE_LANES_MAX 130000
+#endif
+#ifndef WALL_LANES_MAX
+#define WALL_LANES_MAX 60000
+#endif
+
 // integrator + phase change (cryo_phase.cu)
 __global__ void k_kick_drift(Params P, View V, int continuity, int tvf);
 enum { KICK_SOURCES = 1, KICK_HEAT = 2 };
 __global__ void k_kick(Params P, View V, int flags);
 __global__ void k_pc_sources(Params P, View V);
-__global__ void k_pc_normalize(Params P, View V, Reduce R, int sums);
-__global__ void k_pc_apply(Params P, View V, int gated);
+template <int L>
+__global__ void k_pc_normalize(Params P, View V, int gated);
+template <int L>
+__global__ void k_pc_apply(Params P, View V, Reduce R, int gated);
+template <int L>
 __global__ void k_rebalance1(Params P, View V, int gated);
 __global__ void k_rebalance2_mark(Params P, View V, Reduce R, uint32_t* flag, int rebalance, int gated);
 __global__ void k_split(Params P, View V, Reduce R, const uint32_t* flag, int gated);

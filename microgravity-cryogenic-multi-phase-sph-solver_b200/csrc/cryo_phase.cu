@@ -118,79 +118,118 @@ __global__ void __launch_bounds__(kBlock) k_pc_sources(Params P, View V) {
   PARTICLE_LOOP(i, n) pc_source_one(P, V, i, dyn->T_sat, dyn->dt, V.xp[i], false);
 }
 
-// phase_change_normalize (phase_change.cu:139-172); with `sums` (step mode)
-// the FP64 bookkeeping of sph_solver.cu:550-552 (sum_phase_change,
-// count_merges) is reduced in the same pass and added to the cumulative
-// counters.  Step mode is skipped while relax freezes phase change.
-__global__ void __launch_bounds__(kBlock) k_pc_normalize(Params P, View V, Reduce R, int sums) {
-  __shared__ double sh[3 * kBlock / 32];
-  DynState* dyn = V.dyn;
-  if (sums && !dyn->phase_change_on) return;
-  const int n = dyn->n;
-  const int nch = num_chunks(n);
-  const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;
-  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
-    const int i = c * kChunk + threadIdx.x;
-    double s[3] = {0.0, 0.0, 0.0};
-    if (i < n && owned(own_lo, own_hi, n_sorted, i)) {  // a slab skips its ghosts
-      const float4 xpi = V.xp[i];
-      const int fl = fl_of(xpi);
-      if (fl & kSource) {
-        const int target = (fl & kTargetVapor) ? kVapor : kLiquid;
-        float wsum = 0.0f, wr_max = 0.0f;
-        for_each_nbr(P, V, i, xyz(xpi), [&](int j, float4 xj, V3, float r2) {
-          if (j == i || ph_of(xj) != target || (fl_of(xj) & kDying)) return;
-          const float w = kernel_W(P, sqrtf(r2));
-          const float4 mr = __ldg(V.mrps + j);
-          const float rhoj = mr.y;
-          wsum += (mr.x / rhoj) * w;
-          const float wr = w / rhoj;
-          wr_max = wr > wr_max ? wr : wr_max;
-        });
-        float4 pc = V.pc[i];
-        pc.z = wsum;
-        if (!(wsum > 0.0f)) {
-          pc.x = 0.0f;
-        } else if (target == kVapor && P.pc_density_limit > 0.0f && !(fl & kDying) && wr_max > 0.0f) {
-          const float cap = P.pc_density_limit * wsum / wr_max;
-          if (pc.x > cap) pc.x = cap;
-        }
-        V.pc[i] = pc;
-        if (!(fl & kDying)) {
-          if (fl & kTargetVapor) s[0] = (double)pc.x;
-          else s[1] = (double)pc.x;
-        } else if (pc.x > 0.0f) {
-          s[2] = 1.0;
-        }
-      }
-    }
-    if (sums) publish_chunk<3>(R, c, s, sh);
-  }
-  if (sums && last_block(R.ticket)) {
-    const double ev = block_sum_partials(R, 0, nch);
-    const double co = block_sum_partials(R, 1, nch);
-    const double me = block_sum_partials(R, 2, nch);
-    if (threadIdx.x == 0) {
-      dyn->evaporated += ev;
-      dyn->condensed += co;
-      dyn->merges += (int)me;
-    }
-  }
-}
-
-// phase_change_apply (phase_change.cu:174-215)
-__global__ void __launch_bounds__(kBlock) k_pc_apply(Params P, View V, int gated) {
+// phase_change_normalize (phase_change.cu:139-172).  gated (step mode):
+// skipped while relax freezes phase change.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_pc_normalize(Params P, View V, int gated) {
   const DynState* dyn = V.dyn;
   if (gated && !dyn->phase_change_on) return;
   const int n = dyn->n;
-  const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;  // a slab skips its ghosts
-  PARTICLE_LOOP(i, n) {
-    if (!owned(own_lo, own_hi, n_sorted, i)) continue;
-    const float4 xpi = V.xp[i];
-    const int ph = ph_of(xpi);
-    if (!is_fluid(ph)) continue;
+  const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;
+  const int sub = threadIdx.x % L;
+  const int step = gridDim.x * (kBlock / L);
+  for (int i0 = blockIdx.x * (kBlock / L) + (threadIdx.x & ~31) / L; i0 < n; i0 += step) {
+    const int i = i0 + (threadIdx.x & 31) / L;
+    const bool mine = i < n && owned(own_lo, own_hi, n_sorted, i);  // a slab skips its ghosts
+    const float4 xpi = mine ? V.xp[i] : make_float4(0, 0, 0, 0);
     const int fl = fl_of(xpi);
-    float4 mr = V.mrps[i];
+    const bool source = mine && (fl & kSource);
+    if (L == 1 ? !source : !__any_sync(0xffffffffu, source)) continue;
+    const int target = (fl & kTargetVapor) ? kVapor : kLiquid;
+    const V3 xi = xyz(xpi);
+    float wsum = 0.0f, wr_max = 0.0f;
+    auto usable = [&](int j, float4 xj) { return j != i && ph_of(xj) == target && !(fl_of(xj) & kDying); };
+    if constexpr (L == 1) {
+      for_each_nbr(P, V, i, xi, [&](int j, float4 xj, V3, float r2) {
+        if (!usable(j, xj)) return;
+        const float w = kernel_W(P, sqrtf(r2));
+        const float4 mr = __ldg(V.mrps + j);
+        const float rhoj = mr.y;
+        wsum += (mr.x / rhoj) * w;
+        const float wr = w / rhoj;
+        wr_max = wr > wr_max ? wr : wr_max;
+      });
+    } else {
+      NbrRounds<L> nbrs(P, V, i, xi, sub, source);
+      float sw[1] = {0.0f};
+      while (__any_sync(0xffffffffu, nbrs.more())) {
+        float4 xj;
+        const int j = nbrs.take(xj);
+        float tw[1] = {0.0f};
+        const bool use = j >= 0 && usable(j, xj);
+        if (use) {
+          const float w = kernel_W(P, sqrtf(norm2(xi - xyz(xj))));
+          const float4 mr = __ldg(V.mrps + j);
+          const float rhoj = mr.y;
+          tw[0] = (mr.x / rhoj) * w;
+          const float wr = w / rhoj;
+          wr_max = wr > wr_max ? wr : wr_max;
+        }
+        if (__any_sync(0xffffffffu, use)) add_terms<L>(sw, tw);
+      }
+      wsum = sw[0];
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, wr_max, o);
+        wr_max = other > wr_max ? other : wr_max;
+      }
+      if (!source || sub != 0) continue;
+    }
+    float4 pc = V.pc[i];
+    pc.z = wsum;
+    if (!(wsum > 0.0f)) {
+      pc.x = 0.0f;
+    } else if (target == kVapor && P.pc_density_limit > 0.0f && !(fl & kDying) && wr_max > 0.0f) {
+      const float cap = P.pc_density_limit * wsum / wr_max;
+      if (pc.x > cap) pc.x = cap;
+    }
+    V.pc[i] = pc;
+  }
+}
+template __global__ void k_pc_normalize<1>(Params, View, int);
+template __global__ void k_pc_normalize<PASS_LANES>(Params, View, int);
+
+// phase_change_apply (phase_change.cu:174-215).  In step mode (gated) the FP64
+// bookkeeping of sph_solver.cu:550-552 (sum_phase_change, count_merges) is
+// reduced in the same launch from the normalised transfers, which this pass
+// only reads, and added to the cumulative counters.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_pc_apply(Params P, View V, Reduce R, int gated) {
+  __shared__ double sh[3 * kBlock / 32];
+  DynState* dyn = V.dyn;
+  if (gated && !dyn->phase_change_on) return;
+  const int n = dyn->n;
+  const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;  // a slab skips its ghosts
+  const int nch = num_chunks(n);
+  if (gated)
+    for (int c = blockIdx.x; c < nch; c += gridDim.x) {
+      const int i = c * kChunk + threadIdx.x;
+      double s[3] = {0.0, 0.0, 0.0};
+      if (i < n && owned(own_lo, own_hi, n_sorted, i)) {
+        const int fl = fl_of(V.xp[i]);
+        if (fl & kSource) {
+          const float out_m = V.pc[i].x;
+          if (!(fl & kDying)) {
+            if (fl & kTargetVapor) s[0] = (double)out_m;
+            else s[1] = (double)out_m;
+          } else if (out_m > 0.0f) {
+            s[2] = 1.0;
+          }
+        }
+      }
+      publish_chunk<3>(R, c, s, sh);
+    }
+  const int sub = threadIdx.x % L;
+  const int step = gridDim.x * (kBlock / L);
+  for (int i0 = blockIdx.x * (kBlock / L) + (threadIdx.x & ~31) / L; i0 < n; i0 += step) {
+    const int i = i0 + (threadIdx.x & 31) / L;
+    const bool mine = i < n && owned(own_lo, own_hi, n_sorted, i);
+    const float4 xpi = mine ? V.xp[i] : make_float4(0, 0, 0, 0);
+    const int ph = mine ? ph_of(xpi) : kDead;
+    const bool fluid = is_fluid(ph);
+    if (L == 1 ? !fluid : !__any_sync(0xffffffffu, fluid)) continue;
+    const int fl = fl_of(xpi);
+    const float4 mr = fluid ? V.mrps[i] : make_float4(1, 1, 1, 1);
     const float mi = mr.x;
     const float Vi = mi / mr.y;
     float in_m = 0.0f, in_H = 0.0f;
@@ -198,20 +237,42 @@ __global__ void __launch_bounds__(kBlock) k_pc_apply(Params P, View V, int gated
     // nothing (a slab's ghosts are flagged by their owners: no marks there)
     const bool receives = !(fl & kDying) && (!gated || !P.use_lists || P.slab ||
                                              (V.cell_kinds[cell_index(P, xyz(xpi))] & kCellNearSource));
-    if (receives) {
-      for_each_nbr(P, V, i, xyz(xpi), [&](int j, float4 xj, V3, float r2) {
-        // only flagged sources carry out_m > 0 (pc_source_one), so the
-        // others are passed over without reading their pc record
-        if (j == i || !(fl_of(xj) & kSource)) return;
-        const float4 pcj = __ldg(V.pc + j);
-        const float om = pcj.x;
-        if (!(om > 0.0f)) return;
-        const int target = (fl_of(xj) & kTargetVapor) ? kVapor : kLiquid;
-        if (target != ph) return;
-        const float share = om * Vi * kernel_W(P, sqrtf(r2)) / pcj.z;
-        in_m += share;
-        in_H += share * pcj.y;
-      });
+    // only flagged sources carry out_m > 0 (pc_source_one), so the
+    // others are passed over without reading their pc record
+    auto is_source = [&](int j, float4 xj) { return j != i && (fl_of(xj) & kSource); };
+    auto share_of = [&](int j, float4 xj, float r2, float& share, float& enthalpy) {
+      const float4 pcj = __ldg(V.pc + j);
+      const float om = pcj.x;
+      if (!(om > 0.0f)) return false;
+      const int target = (fl_of(xj) & kTargetVapor) ? kVapor : kLiquid;
+      if (target != ph) return false;
+      share = om * Vi * kernel_W(P, sqrtf(r2)) / pcj.z;
+      enthalpy = share * pcj.y;
+      return true;
+    };
+    if constexpr (L == 1) {
+      if (receives) {
+        for_each_nbr(P, V, i, xyz(xpi), [&](int j, float4 xj, V3, float r2) {
+          float share, enthalpy;
+          if (!is_source(j, xj) || !share_of(j, xj, r2, share, enthalpy)) return;
+          in_m += share;
+          in_H += enthalpy;
+        });
+      }
+    } else {
+      const V3 xi = xyz(xpi);
+      NbrRounds<L> nbrs(P, V, i, xi, sub, fluid && receives);
+      float s[2] = {0.0f, 0.0f};
+      while (__any_sync(0xffffffffu, nbrs.more())) {
+        float4 xj;
+        const int j = nbrs.take(xj);
+        float t[2] = {0.0f, 0.0f};
+        const bool gives = j >= 0 && is_source(j, xj) && share_of(j, xj, norm2(xi - xyz(xj)), t[0], t[1]);
+        if (__any_sync(0xffffffffu, gives)) add_terms<L>(s, t);
+      }
+      in_m = s[0];
+      in_H = s[1];
+      if (!fluid || sub != 0) continue;
     }
     const float4 pci = V.pc[i];
     const float om_i = pci.x;
@@ -228,54 +289,97 @@ __global__ void __launch_bounds__(kBlock) k_pc_apply(Params P, View V, int gated
     V.vT[i] = vT;
     V.mrps[i].x = m_new;
   }
+  if (gated && last_block(R.ticket)) {
+    const double ev = block_sum_partials(R, 0, nch);
+    const double co = block_sum_partials(R, 1, nch);
+    const double me = block_sum_partials(R, 2, nch);
+    if (threadIdx.x == 0) {
+      dyn->evaporated += ev;
+      dyn->condensed += co;
+      dyn->merges += (int)me;
+    }
+  }
 }
+template __global__ void k_pc_apply<1>(Params, View, Reduce, int);
+template __global__ void k_pc_apply<PASS_LANES>(Params, View, Reduce, int);
 
 // rebalance_vapor_mass, pass 1 (phase_change.cu:223-250).  The momentum
 // exchange goes to ns (as in the reference).
+template <int L>
 __global__ void __launch_bounds__(kBlock) k_rebalance1(Params P, View V, int gated) {
   const DynState* dyn = V.dyn;
   if (gated && !dyn->phase_change_on) return;
   const int n = dyn->n;
   const float beta = P.vapor_rebalance;
   const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;  // a slab skips its ghosts
-  PARTICLE_LOOP(i, n) {
-    if (!owned(own_lo, own_hi, n_sorted, i)) continue;
-    const float4 xpi = V.xp[i];
-    const float kap = V.ns4[i].w;
-    const float wn = V.pc[i].z;
-    if (ph_of(xpi) != kVapor) {
+  const int sub = threadIdx.x % L;
+  const int step = gridDim.x * (kBlock / L);
+  for (int i0 = blockIdx.x * (kBlock / L) + (threadIdx.x & ~31) / L; i0 < n; i0 += step) {
+    const int i = i0 + (threadIdx.x & 31) / L;
+    const bool mine = i < n && owned(own_lo, own_hi, n_sorted, i);
+    if (L == 1 && !mine) continue;
+    const float4 xpi = mine ? V.xp[i] : make_float4(0, 0, 0, 0);
+    const bool vapour = mine && ph_of(xpi) == kVapor;
+    const float kap = mine ? V.ns4[i].w : 0.0f;
+    const float wn = mine ? V.pc[i].z : 0.0f;
+    if (mine && !vapour && sub == 0) {
       V.pc[i] = make_float4(0.0f, 0.0f, wn, 0.0f);
       V.ns4[i] = make_float4(0.0f, 0.0f, 0.0f, kap);
-      continue;
     }
-    const float mi = V.mrps[i].x;
-    const float4 vTi = V.vT[i];
+    if (L == 1 ? !vapour : !__any_sync(0xffffffffu, vapour)) continue;
+    const float mi = vapour ? V.mrps[i].x : 0.0f;
+    const float4 vTi = vapour ? V.vT[i] : make_float4(0, 0, 0, 0);
     const float hi = specific_enthalpy(P, kVapor, vTi.w);
     const V3 vi = xyz(vTi);
-    float dm = 0.0f, dH = 0.0f;
-    V3 dP{0, 0, 0};
-    for_each_nbr_pf(P, V, i, xyz(xpi), V.mrps, [&](int j, float4 xj, V3, float r2, const float4& mrj) {
-      if (j == i || ph_of(xj) != kVapor) return;
-      const float mj = mrj.x;
-      // equal masses give flow = +0, and every sum below gains a zero that
-      // leaves it as it is
-      if (mj == mi) return;
+    float s[5] = {0, 0, 0, 0, 0};  // mass, enthalpy, momentum
+    // equal masses give flow = +0, and every sum below gains a zero that
+    // leaves it as it is
+    auto flows = [&](int j, float r2, float mj, float (&t)[5]) {
       const float flow = beta * P.vol0 * kernel_W(P, sqrtf(r2)) * (mj - mi);
       const bool from_j = flow > 0.0f;
-      dm += flow;
+      float h = hi;
+      V3 v = vi;
       if (from_j) {
         const float4 vTj = __ldg(V.vT + j);
-        dH += flow * specific_enthalpy(P, kVapor, vTj.w);
-        dP += xyz(vTj) * flow;
-      } else {
-        dH += flow * hi;
-        dP += vi * flow;
+        h = specific_enthalpy(P, kVapor, vTj.w);
+        v = xyz(vTj);
       }
-    });
-    V.pc[i] = make_float4(dm, dH, wn, 0.0f);
-    V.ns4[i] = f4(dP, kap);
+      t[0] = flow;
+      t[1] = flow * h;
+      t[2] = v.x * flow;
+      t[3] = v.y * flow;
+      t[4] = v.z * flow;
+    };
+    if constexpr (L == 1) {
+      for_each_nbr_pf(P, V, i, xyz(xpi), V.mrps, [&](int j, float4 xj, V3, float r2, const float4& mrj) {
+        if (j == i || ph_of(xj) != kVapor || mrj.x == mi) return;
+        float t[5];
+        flows(j, r2, mrj.x, t);
+        add_terms<1>(s, t);
+      });
+    } else {
+      const V3 xi = xyz(xpi);
+      NbrRounds<L> nbrs(P, V, i, xi, sub, vapour);
+      while (__any_sync(0xffffffffu, nbrs.more())) {
+        float4 xj;
+        const int j = nbrs.take(xj);
+        float t[5] = {0, 0, 0, 0, 0};
+        bool differs = false;
+        if (j >= 0 && j != i && ph_of(xj) == kVapor) {
+          const float mj = __ldg(V.mrps + j).x;
+          differs = mj != mi;
+          if (differs) flows(j, norm2(xi - xyz(xj)), mj, t);
+        }
+        if (__any_sync(0xffffffffu, differs)) add_terms<L>(s, t);
+      }
+      if (!vapour || sub != 0) continue;
+    }
+    V.pc[i] = make_float4(s[0], s[1], wn, 0.0f);
+    V.ns4[i] = make_float4(s[2], s[3], s[4], kap);
   }
 }
+template __global__ void k_rebalance1<1>(Params, View, int);
+template __global__ void k_rebalance1<PASS_LANES>(Params, View, int);
 
 // rebalance_vapor_mass, pass 2 (phase_change.cu:252-267), then
 // mark_heavy_particles (phase_change.cu:270-279) with the per-chunk counts of

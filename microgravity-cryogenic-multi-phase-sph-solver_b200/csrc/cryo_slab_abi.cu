@@ -499,7 +499,7 @@ int cryo_slabs_set_particles(cryo_slabs* s, const cryo_host_particles_t* p, cons
     const int R = G.count();
     cryo_ctx* c0 = G.slabs[0];
     CK(cudaSetDevice(c0->device));
-    c0->begin_load(1, vap, lo, hi);  // the grid the whole tank has
+    c0->begin_load(1, 1, vap, lo, hi);  // the grid the whole tank has
     const Params P0 = c0->P;
     std::vector<int> layer(n);
     std::vector<long long> counts(P0.nz, 0);
@@ -524,7 +524,8 @@ int cryo_slabs_set_particles(cryo_slabs* s, const cryo_host_particles_t* p, cons
       for (int i = 0; i < n; ++i)
         if (layer[i] >= z0 && layer[i] < z1) idx.push_back(i);
       const int m = (int)idx.size();
-      c->begin_load(std::max(m, 1), vap, lo, hi);
+      const int fluid = (int)std::count_if(idx.begin(), idx.end(), [&](int i) { return is_fluid(p->phase[i]); });
+      c->begin_load(std::max(m, 1), fluid, vap, lo, hi);
       c->P.slab_z0 = G.zb[r];  // the passes run over owned particles only
       c->P.slab_z1 = G.zb[r + 1];
       std::vector<float4> xp(m), vT(m), vt(m), nrm(m), mrps(m);

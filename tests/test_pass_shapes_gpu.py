@@ -1,5 +1,6 @@
-"""The cell sort and the neighbour-list build at the sizes where a change of
-launch shape or a remainder can go wrong, bit for bit."""
+"""The cell sort, the neighbour-list build and the neighbour passes at the
+sizes where a change of launch shape or a remainder can go wrong.  Every
+comparison is bit for bit: the shapes add the same terms in the same order."""
 import numpy as np
 import pytest
 
@@ -87,3 +88,86 @@ def test_lists_of_a_large_tank(cuda_device):
                      "phase": p["phase"], "nrm": p["normal"]}, lo, hi)
     g.run_pass("grid_build")
     assert_stored_equal_scan(g, g.field("phase"))
+
+
+@pytest.mark.parametrize("phase_change", [0, 1])
+def test_more_neighbours_than_the_lists_hold(cuda_device, phase_change):
+    """Particles with over 128 neighbours search the cells instead; a tank in
+    which some do equals one stepped without lists."""
+    p = cloud(900, 3, dense=0)
+    p["x"][:400] = np.random.default_rng(1).uniform((0.1, 0.1, 0.1), (0.13, 0.13, 0.13), (400, 3)).astype(np.float32)
+    p["phase"][100:160] = 1
+    p["phase"][160:220] = 2
+    p["T"][:100] = 380.0
+    cfg = cabi.py_config(dx=0.012, gravity=(0, 0, -1.0), velocity_scale=1.0, thermo_mode=1, heater_power=3.0,
+                         phase_change=phase_change, fixed_dt=1e-6)
+    out = []
+    for lists in (1, 0):
+        g = cabi.Context(cfg, cabi.py_fluid(cabi.FLUID_H2O))
+        g.set_neighbor_mode(lists)
+        g.set_particles(p, LO, HI)
+        g.step(3)
+        if lists:
+            assert g.neighbor_lists()[0].max() > 128
+        out.append({f: g.field(f) for f in ("x", "v", "rho", "T", "m", "p", "a", "sigma", "nrm", "kappa", "fw", "mw")})
+    for f in out[0]:
+        assert np.array_equal(out[0][f].view(np.uint32), out[1][f].view(np.uint32)), f
+
+
+def small_tanks():
+    """Two-phase and free-surface tanks over the options the passes branch on."""
+    ln2, h2o = cs.FluidProperties.liquid_nitrogen, cs.FluidProperties.water
+
+    def make(geo, fluid, fill, seed, **kw):
+        cfg = cs.SolverConfig()
+        cfg.dx = 0.004
+        for k, v in kw.items():
+            cur = getattr(cfg, k)
+            setattr(cfg, k, type(cur)(v) if hasattr(cur, "value") else v)
+        s = cs.Solver(cfg, fluid)
+        s.build_tank(geo, fill)
+        s.jitter_fluid(0.0002, seed)
+        return s
+
+    def fill(fraction, dT=0.0, vapour=True):
+        f = cs.FillSpec()
+        f.fill_fraction = fraction
+        f.include_vapor = vapour
+        if dT:
+            f.T_liquid = ln2().T_sat + dT
+        return f
+
+    return [
+        lambda: make(cs.BoxTank(0.03, 0.03, 0.03), ln2(), fill(0.5, 3.0), 1, gravity=(0.1, 0, -0.5)),
+        lambda: make(cs.CylinderTank(0.03, 0.06), ln2(), fill(0.4, 2.0), 2, heater_power=20.0, thermo_mode=1,
+                     wetting_model=2),
+        lambda: make(cs.SphereTank(0.03), ln2(), fill(0.6), 3, csf_balanced=True, sps_turbulence=True,
+                     transport_stress=True, wall_thermal_bc=1, thermo_mode=1),
+        lambda: make(cs.BoxTank(0.04, 0.03, 0.03), h2o(), fill(0.5, vapour=False), 4, surface_tension=2, thermal=False,
+                     phase_change=False, velocity_scale=0.5, gravity=(0, 0, -1.0)),
+        lambda: make(cs.BoxTank(0.04, 0.03, 0.03), h2o(), fill(0.5, vapour=False), 5, surface_tension=0, thermal=False,
+                     phase_change=False, density_mode=1, velocity_scale=0.5, gravity=(0, 0, -1.0), no_slip=False),
+    ]
+
+
+def test_lanes_and_threads_give_the_same_bits(cuda_device):
+    """A small tank alone steps with lanes sharing its particles; beside a
+    tank that fills the chip it steps with a thread per particle."""
+    water, p, (lo, hi) = big_tank()
+    cfg = cs.SolverConfig()
+    cfg.dx = 0.004
+    filler = cs.Solver(cfg, water)
+    filler.set_particles(p["position"], p["mass"], p["density"], p["temperature"], p["phase"], domain_lo=lo,
+                         domain_hi=hi, normal=p["normal"], flags=p["flags"])
+    crowd, alone = cs.Ensemble(0), [make() for make in small_tanks()]
+    beside = [make() for make in small_tanks()]
+    crowd.add(filler)
+    for s in beside:
+        crowd.add(s)
+    crowd.run_steps(6)
+    for a, b in zip(alone, beside):
+        a.run_steps(6)
+        pa, pb = a.particles(), b.particles()
+        for k in pa:
+            assert np.array_equal(np.asarray(pa[k]).view(np.uint8), np.asarray(pb[k]).view(np.uint8)), k
+        assert a.diagnostics().as_dict() == b.diagnostics().as_dict()
