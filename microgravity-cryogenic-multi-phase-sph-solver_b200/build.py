@@ -35,7 +35,7 @@ NVCC_FLAGS = [
 # cryo_physics.cu again for the fast field arithmetic: FMA contraction and
 # approximate division / square root (denormals kept).
 FAST_FIELD_FLAGS = [f for f in NVCC_FLAGS if f != "-fmad=false"] + [
-    "-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-DCRYO_FIELD_NS=fast"]
+    "-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-DCRYO_FIELD_NS=fast", "-DCRYO_FIELD_FAST=1"]
 LIB = os.path.join(HERE, "libcryosph_b200.so")
 
 

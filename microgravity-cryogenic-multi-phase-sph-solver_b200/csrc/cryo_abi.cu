@@ -256,6 +256,11 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
   const int GF = forces_blocks();
   const bool laned = rate_lanes(loaded_fluid, FORCES_LANES_MAX);
   const int GL = lane_blocks(FORCES_LANED_BLOCK);
+  // The instances with the rarer options compiled out (cryo_physics.cu).  In
+  // the fast arithmetic only four sets have one: those where every sum is known
+  // to keep the general instance's contraction, hence its bits.
+  const bool common = P.ktype != CRYO_KERNEL_CUBIC && !P.sps && !(P.tvf && P.tvf_stress) &&
+                      !P.csf_balanced && P.wall_bc != CRYO_WALL_ISOTHERMAL;
   int what = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
   if (P.csf_active) what |= FORCE_CSF;
   if (P.st_model == CRYO_ST_AKINCI) what |= FORCE_AKINCI;
@@ -278,20 +283,35 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
     }
     return;
   }
+#define FORCES_CASE_COMMON(W)                                                                  \
+  case W:                                                                                      \
+    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
+    else if (common) FIELD_LAUNCH(k_forces_t<(W) | FORCE_COMMON>, GF, FORCES_BLOCK, P, V, W);  \
+    else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);                               \
+    break;
+#define FORCES_CASE_COMMON_EXACT(W)                                                            \
+  case W:                                                                                      \
+    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
+    else if (common && !fast_fields)                                                           \
+      LAUNCH(exact::k_forces_t<(W) | FORCE_COMMON>, GF, FORCES_BLOCK, P, V, W);                \
+    else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);                               \
+    break;
   switch (what) {
-    FORCES_CASE(FORCE_BASE)
-    FORCES_CASE(FORCE_BASE | FORCE_THERMAL)
-    FORCES_CASE(FORCE_BASE | FORCE_DRHO)
-    FORCES_CASE(FORCE_BASE | FORCE_DRHO | FORCE_THERMAL)
+    FORCES_CASE_COMMON(FORCE_BASE)
+    FORCES_CASE_COMMON(FORCE_BASE | FORCE_DRHO)
+    FORCES_CASE_COMMON(FORCE_BASE | FORCE_CSF)
+    FORCES_CASE_COMMON(FORCE_BASE | FORCE_CSF | FORCE_THERMAL)
+    FORCES_CASE_COMMON_EXACT(FORCE_BASE | FORCE_THERMAL)
+    FORCES_CASE_COMMON_EXACT(FORCE_BASE | FORCE_DRHO | FORCE_THERMAL)
+    FORCES_CASE_COMMON_EXACT(FORCE_BASE | FORCE_CSF | FORCE_DRHO)
+    FORCES_CASE_COMMON_EXACT(FORCE_BASE | FORCE_CSF | FORCE_DRHO | FORCE_THERMAL)
     FORCES_CASE(FORCE_BASE | FORCE_AKINCI)
     FORCES_CASE(FORCE_BASE | FORCE_AKINCI | FORCE_THERMAL)
     FORCES_CASE(FORCE_BASE | FORCE_AKINCI | FORCE_DRHO)
     FORCES_CASE(FORCE_BASE | FORCE_AKINCI | FORCE_DRHO | FORCE_THERMAL)
-    FORCES_CASE(FORCE_BASE | FORCE_CSF)
-    FORCES_CASE(FORCE_BASE | FORCE_CSF | FORCE_THERMAL)
-    FORCES_CASE(FORCE_BASE | FORCE_CSF | FORCE_DRHO)
-    FORCES_CASE(FORCE_BASE | FORCE_CSF | FORCE_DRHO | FORCE_THERMAL)
 #undef FORCES_CASE
+#undef FORCES_CASE_COMMON
+#undef FORCES_CASE_COMMON_EXACT
     default: FIELD_LAUNCH(k_forces_t<-1>, GF, FORCES_BLOCK, P, V, what);
   }
   slab_point(SLAB_FORCES, s);

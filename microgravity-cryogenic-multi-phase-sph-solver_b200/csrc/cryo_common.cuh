@@ -293,10 +293,11 @@ __host__ __device__ inline float kernel_W(const Params& P, float r) {
   const float t2 = t * t;
   return P.knorm * t2 * t2 * (2.0f * q + 1.0f);
 }
+template <bool WENDLAND = false>  // known to be the Wendland kernel
 __host__ __device__ inline float kernel_dWdr(const Params& P, float r) {
   const float q = r * P.inv_h;
   if (q >= 2.0f) return 0.0f;
-  if (P.ktype == CRYO_KERNEL_CUBIC) {
+  if (!WENDLAND && P.ktype == CRYO_KERNEL_CUBIC) {
     if (q < 1.0f) return P.knorm * P.inv_h * (-3.0f * q + 2.25f * q * q);
     const float t = 2.0f - q;
     return P.knorm * P.inv_h * -0.75f * t * t;
@@ -483,6 +484,13 @@ __device__ inline void for_each_nbr(const Params& P, const View& V, int i, V3 xi
   } else {
     for_each_neighbor(P, V.cell_begin, V.xp, xi, f);
   }
+}
+
+// The last entry of a list with an odd count, else -1.
+__device__ inline int left_over_nbr(const Params& P, const View& V, int i) {
+  const int c = P.use_lists ? __ldg(V.nbr_cnt + i) : 0;
+  if (!(c & 1) || c > kMaxNbr) return -1;
+  return __ldg(V.nbr + (size_t)((c - 1) / kNbrChunk) * V.capacity * kNbrChunk + (size_t)i * kNbrChunk + (c - 1) % kNbrChunk);
 }
 
 // for_each_nbr for passes with little work per neighbour: the loop takes

@@ -217,7 +217,8 @@ __global__ void k_nbr_fill(Params P, View V, int stored, const long long* offset
 // physics (cryo_physics.cu).  Fused rate pass; `what` selects the sub-passes (FORCE_* bits).
 enum { FORCE_TRANSPORT = 1, FORCE_MOMENTUM = 2, FORCE_CSF = 4, FORCE_AKINCI = 8, FORCE_DRHO = 16,
        FORCE_THERMAL = 32, FORCE_MAXIMA = 64, FORCE_THERMAL_ALWAYS = 128,
-       FORCE_TAPE = 256 };  // compile-time only: also store the sums into V.tape
+       FORCE_TAPE = 256,      // compile-time only: also store the sums into V.tape
+       FORCE_COMMON = 512 };  // compile-time only: the rarer options are off (cryo_physics.cu)
 // cryo_physics.cu is compiled twice.  namespace exact: the reference's IEEE
 // single-precision operation sequence (no FMA contraction, IEEE division and
 // square root), bit-identical to its CPU build.  namespace fast: the same
@@ -272,13 +273,20 @@ constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
 #ifndef FORCES_MIN_BLOCKS
 #define FORCES_MIN_BLOCKS 9
 #endif
-// The sub-pass sets with surface tension or heat need ~125 registers; at
-// 8 blocks per SM (4 warps per sub-partition) they run without spilling.
+// The sub-pass sets with surface tension or heat run without spilling at 8
+// blocks per SM (4 warps per sub-partition).  With FORCE_COMMON the fast
+// arithmetic needs fewer registers and takes 10: 778 us against 874 at 1.06 M
+// particles, while the exact one spills there (4235 against 4024 at 4.08 M).
 #ifndef FORCES_MIN_BLOCKS_HEAVY
 #define FORCES_MIN_BLOCKS_HEAVY 8
 #endif
-constexpr int forces_min_blocks(int what) {
-  return (what >= 0 && (what & (FORCE_CSF | FORCE_THERMAL))) ? FORCES_MIN_BLOCKS_HEAVY : FORCES_MIN_BLOCKS;
+#ifndef FORCES_MIN_BLOCKS_FAST
+#define FORCES_MIN_BLOCKS_FAST 10
+#endif
+constexpr int forces_min_blocks(int what, bool fast) {
+  return !(what >= 0 && (what & (FORCE_CSF | FORCE_THERMAL))) ? FORCES_MIN_BLOCKS
+         : fast && (what & FORCE_COMMON)                      ? FORCES_MIN_BLOCKS_FAST
+                                                              : FORCES_MIN_BLOCKS_HEAVY;
 }
 // Neighbour-loop unroll of the force-pass variants with surface tension or
 // heat (the two-phase tanks): 2 takes the 4 M-particle LH2 sphere 3 % faster,
@@ -287,11 +295,12 @@ constexpr int forces_min_blocks(int what) {
 #define FORCES_UNROLL_HEAVY 2
 #endif
 // Neighbour-list build: LIST_LANES lanes per particle up to LIST_LANES_MAX
-// particles, one above (k_build_lists).
+// particles, one above (k_build_lists): lanes 25 us against 41 at 27 k, 81
+// against 68 at 91 k, 93 against 78 at 204 k.
 constexpr int LIST_LANES = 4;
 constexpr int kListPad = 8;  // records the build may load beyond the last particle
 #ifndef LIST_LANES_MAX
-#define LIST_LANES_MAX 300000
+#define LIST_LANES_MAX 60000
 #endif
 // The neighbour passes that come in two shapes, one thread per particle and
 // PASS_LANES lanes per particle, take the second up to these counts (fluid

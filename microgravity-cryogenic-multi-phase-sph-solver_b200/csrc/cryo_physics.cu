@@ -8,6 +8,9 @@
 #ifndef CRYO_FIELD_NS
 #define CRYO_FIELD_NS exact
 #endif
+#ifndef CRYO_FIELD_FAST
+#define CRYO_FIELD_FAST 0
+#endif
 
 namespace cryo {
 namespace CRYO_FIELD_NS {
@@ -367,11 +370,35 @@ __global__ void __launch_bounds__(kBlock) k_smooth_normals(Params P, View V) {
 // (phase_change.cu:31-75) and the dt maxima (sph_solver.cu:59-99, 475-479),
 // in one neighbour loop.  Each sub-pass reads only what the previous passes
 // wrote, never what this pass writes, so fusing keeps the reference's values.
+// Vi^2 + Vj^2 with Vi2 = Vi^2.  In the fast arithmetic the compiler contracts
+// it into either product, differently from one instance of the force pass to
+// the next; the instances with FORCE_COMMON state it (FMA 1: the neighbour's
+// square is the fused one, 2: the particle's own), so that a particle's sums
+// keep the bits of the general instance.
+template <int FMA>
+__device__ inline float sum_squares(float Vi, float Vi2, float Vj) {
+  if (FMA == 1) return __fmaf_rn(Vj, Vj, Vi2);
+  if (FMA == 2) return __fmaf_rn(Vi, Vi, __fmul_rn(Vj, Vj));
+  return Vi2 + Vj * Vj;
+}
+
+// FORCE_COMMON instances: Wendland kernel, no sub-particle stresses, no
+// transport stress, plain CSF, walls not isothermal, known when compiled.  The
+// pass issues instructions all the time (two thirds of its issue slots, DRAM a
+// tenth busy), and each of those options cost a test per pair and registers
+// over the whole loop: without them 4.08 M particles took 4024 us in place of
+// 4718, 1.06 M in the fast arithmetic 778 in place of 1018, the dam of 204 k
+// 128 in place of 152.
 template <int WHAT>
-__global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_forces_t(Params P, View V, int what_rt) {
+__global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIELD_FAST)) k_forces_t(Params P, View V, int what_rt) {
   // WHAT >= 0: the sub-pass set is a compile-time constant (the step path);
   // -1: read at run time (operator-level calls)
-  const int what = WHAT >= 0 ? WHAT : what_rt;
+  const int what = WHAT >= 0 ? WHAT & ~FORCE_COMMON : what_rt;
+  constexpr bool kCommon = WHAT >= 0 && (WHAT & FORCE_COMMON);
+  constexpr bool kStated = CRYO_FIELD_FAST && kCommon;
+  constexpr int kFmaW = kStated ? ((WHAT & FORCE_CSF) && (WHAT & FORCE_THERMAL) ? 2 : 1) : 0;
+  const bool sps = kCommon ? false : P.sps != 0;
+  const bool csf_balanced = kCommon ? false : P.csf_balanced != 0;
   DynState* dyn = V.dyn;
   const int n = dyn->n;
   const bool thermal = ((what & FORCE_THERMAL) && dyn->thermal_on) || (what & FORCE_THERMAL_ALWAYS);
@@ -380,10 +407,10 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
   const float h = P.h;
   const float eta2 = 0.01f * h * h;
   const float r_guard = 0.6f * P.dx;
-  const bool tvf_stress = P.tvf && P.tvf_stress;
+  const bool tvf_stress = kCommon ? false : P.tvf && P.tvf_stress;
   const float inv_gamma = 1.0f / P.tait_gamma;
   const float csf_coeff = 2.0f * P.sigma / (P.rho0[0] + P.rho0[1]);
-  const bool iso_walls = P.wall_bc == CRYO_WALL_ISOTHERMAL;
+  const bool iso_walls = kCommon ? false : P.wall_bc == CRYO_WALL_ISOTHERMAL;
   const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;
   float vmax_l = 0.0f, amax_l = 0.0f, tv_l = 0.0f, sr_l = 0.0f, nut_l = 0.0f;
 
@@ -422,7 +449,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
     const float Vi = mi / rhoi;
     const float Vi2 = Vi * Vi;
     const float ci = sound_speed(P, ph, Ti);
-    const float etai = P.mu[pi_idx] + (P.sps ? rhoi * V.nu_t[i] : 0.0f);
+    const float etai = P.mu[pi_idx] + (sps ? rhoi * V.nu_t[i] : 0.0f);
     const float alpha_i = ph == kVapor ? P.alpha_av_vap : P.alpha_av;
     // harmonic viscosity per neighbour phase (navier_stokes.cu:190-196),
     // evaluated once per particle when it does not vary per neighbour
@@ -432,7 +459,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
     // neighbour's phase would live in local memory, a load on every pair's
     // dependent chain)
     float eta_pair0 = 0.0f, eta_pair1 = 0.0f;
-    if (!P.sps) {
+    if (!sps) {
       auto harmonic = [&](float etaj) {
         const float eta_sum = etai + etaj;
         return eta_sum > 0.0f ? 2.0f * etai * etaj / eta_sum : 0.0f;
@@ -480,10 +507,18 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
 
     constexpr int kUnroll = (FORCES_UNROLL_HEAVY > 1 && WHAT >= 0 && (WHAT & (FORCE_CSF | FORCE_THERMAL)))
                                 ? FORCES_UNROLL_HEAVY : 1;
+    // (of an odd number of neighbours the last one, which the loop unrolled by
+    // two leaves over, has its square fused the other way)
+    int j_left = -1;
+    if (kStated && kUnroll == 2 && do_T) j_left = left_over_nbr(P, V, i);
+    auto sumT_squares = [&](int j, float Vj) {
+      if (!kStated) return VT_i2 + Vj * Vj;
+      return kUnroll == 2 && j == j_left ? sum_squares<1>(VT_i, VT_i2, Vj) : sum_squares<2>(VT_i, VT_i2, Vj);
+    };
     for_each_nbr<kUnroll>(P, V, i, xi, [&](int j, float4 xj, V3 rij, float r2) {
       if (j == i) return;
       const float r = sqrtf(r2);
-      const float dW = kernel_dWdr(P, r);
+      const float dW = kernel_dWdr<kCommon>(P, r);
       const bool separated = r > 1e-12f * h;
       const V3 gw = separated ? rij * (dW / r) : V3{0, 0, 0};  // == kernel_gradW
       const int phj = ph_of(xj);
@@ -499,12 +534,12 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
             rho_w = P.rho0[0] * powf(ratio > 0.5f ? ratio : 0.5f, inv_gamma);
           }
           const float Vj = rho_w > 0.0f ? VT_i * rhoi / rho_w : VT_i;
-          sumT += gw * (VT_i2 + Vj * Vj);
+          sumT += gw * sumT_squares(j, Vj);
         }
         if (what & FORCE_MOMENTUM) {
           const V3 f_before = force, a_before = acc_av;
           const float Vj = P.vol0;
-          const float vsum = Vi2 + Vj * Vj;
+          const float vsum = sum_squares<kFmaW>(Vi, Vi2, Vj);
           const float pw = ph == kVapor ? vwj.w : mrj.z;
           force -= gw * (vsum * 0.5f * (pi + pw));
           if (tvf_stress) force += vi * (0.5f * vsum * rhoi * dot(dvi, gw));
@@ -548,7 +583,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
       const float mj = mrj.x, rhoj = mrj.y;
       if (do_T) {
         const float Vj = axj.y;
-        sumT += gw * (VT_i2 + Vj * Vj);
+        sumT += gw * sumT_squares(j, Vj);
       }
       const float Vj = axj.x;
       if (what & FORCE_MOMENTUM) {
@@ -561,7 +596,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
           force += Ag * (0.5f * vsum);
         }
         const V3 vij = vi - xyz(vTj);
-        if (P.sps) {
+        if (sps) {
           const float etaj = P.mu[phase_index(phj)] + rhoj * V.nu_t[j];
           const float eta_sum = etai + etaj;
           if (eta_sum > 0.0f && separated) {
@@ -589,7 +624,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
           num += Vj * dot(ni - nj, gwC);
           den += Vj * r * (-dW);
         }
-        if (P.csf_balanced) {
+        if (csf_balanced) {
           const float cj = phj == kLiquid ? 1.0f : 0.0f;
           G += gwC * ((Vi * Vi + Vj * Vj) * (rhoj * ciC + rhoi * cj) / (rhoi + rhoj));
         }
@@ -647,8 +682,8 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
         const float kappa = den > 0.0f ? 3.0f * num / den : 0.0f;
         ns4.w = kappa;
         if (P.wetting_model != 0) acc += xyz(V.vwp[i]);
-        if (P.csf_balanced) acc += G * (P.sigma * kappa / mi);
-        else acc += xyz(nrmi) * (csf_coeff * kappa);
+        if (csf_balanced) acc += G * (P.sigma * kappa / mi);
+        else acc += xyz(kCommon ? V.nrm[i] : nrmi) * (csf_coeff * kappa);
       }
       V.ns4[i] = ns4;
     }
@@ -668,7 +703,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
       const float aa = norm(acc), bb = norm(ab);
       amax_l = fmaxf(amax_l, aa > bb ? aa : bb);
       if (ph == kVapor) tv_l = fmaxf(tv_l, Ti);
-      if (P.sps) nut_l = fmaxf(nut_l, V.nu_t[i]);
+      if (sps) nut_l = fmaxf(nut_l, V.nu_t[i]);
     }
   }
   if (what & FORCE_MAXIMA) {
@@ -682,7 +717,7 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_force
       atomic_max_pos(&dyn->a_max, amax_l);
       if (P.has_vapor) atomic_max_pos(&dyn->Tv_max, tv_l);
       atomic_max_pos(&dyn->spacing_ratio, sr_l);
-      if (P.sps) atomic_max_pos(&dyn->nu_t_max, nut_l);
+      if (sps) atomic_max_pos(&dyn->nu_t_max, nut_l);
     }
   }
 }
@@ -701,6 +736,16 @@ template __global__ void k_forces_t<71>(Params, View, int);
 template __global__ void k_forces_t<103>(Params, View, int);
 template __global__ void k_forces_t<87>(Params, View, int);
 template __global__ void k_forces_t<119>(Params, View, int);
+template __global__ void k_forces_t<67 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<83 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<71 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<103 | FORCE_COMMON>(Params, View, int);
+#if !CRYO_FIELD_FAST
+template __global__ void k_forces_t<99 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<115 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<87 | FORCE_COMMON>(Params, View, int);
+template __global__ void k_forces_t<119 | FORCE_COMMON>(Params, View, int);
+#endif
 // taped variants (FORCE_TAPE) of the sub-pass sets the adjoint covers
 template __global__ void k_forces_t<323>(Params, View, int);
 template __global__ void k_forces_t<355>(Params, View, int);

@@ -171,3 +171,39 @@ def test_lanes_and_threads_give_the_same_bits(cuda_device):
         for k in pa:
             assert np.array_equal(np.asarray(pa[k]).view(np.uint8), np.asarray(pb[k]).view(np.uint8)), k
         assert a.diagnostics().as_dict() == b.diagnostics().as_dict()
+
+
+# (options, what takes the force pass off the instance with the rarer options
+# compiled out without changing a value, arithmetics that have such an instance)
+OTHER_ROUTE = [
+    (dict(surface_tension=0, thermal=0, density_mode=0), dict(csf_balanced=1), (0, 1)),
+    (dict(surface_tension=0, thermal=0, density_mode=1, no_slip=0), dict(csf_balanced=1), (0, 1)),
+    (dict(surface_tension=0, thermal=1, density_mode=0), dict(csf_balanced=1), (0,)),
+    (dict(surface_tension=0, thermal=1, density_mode=1), dict(csf_balanced=1), (0,)),
+    (dict(surface_tension=1, thermal=0, density_mode=0), dict(wall_thermal_bc=1), (0, 1)),
+    (dict(surface_tension=1, thermal=0, density_mode=1), dict(wall_thermal_bc=1), (0,)),
+    (dict(surface_tension=1, thermal=1, density_mode=0), dict(sps_turbulence=1, smagorinsky_cs=0.0), (0,)),
+    (dict(surface_tension=1, thermal=1, density_mode=1), dict(sps_turbulence=1, smagorinsky_cs=0.0), (0,)),
+    # all temperatures equal: an isothermal wall exchanges nothing
+    (dict(surface_tension=1, thermal=1, density_mode=0, T=300.0), dict(wall_thermal_bc=1), (0, 1)),
+]
+
+
+@pytest.mark.parametrize("base,other,arithmetics", OTHER_ROUTE)
+def test_force_pass_without_the_rarer_options(cuda_device, base, other, arithmetics):
+    _, p, (lo, hi) = big_tank()
+    base = dict(base)
+    T = np.full(len(p["mass"]), base.pop("T"), np.float32) if "T" in base else p["temperature"]
+    x = p["position"] + np.random.default_rng(5).uniform(-2e-4, 2e-4, p["position"].shape).astype(np.float32)
+    for arithmetic in arithmetics:
+        out = []
+        for extra in ({}, other):
+            g = cabi.Context(cabi.py_config(dx=0.004, gravity=(0, 0, -1.0), phase_change=0, thermo_mode=1,
+                                            transport_velocity=1, **base, **extra), cabi.py_fluid(cabi.FLUID_H2O))
+            g.set_field_arithmetic(arithmetic)
+            g.set_particles({"x": x, "m": p["mass"], "rho": p["density"], "T": T, "phase": p["phase"],
+                             "nrm": p["normal"]}, lo, hi)
+            g.step(2)
+            out.append({f: g.field(f) for f in ("x", "v", "rho", "T", "a", "ab", "drho", "dTdt", "fw", "mw")})
+        for f in out[0]:
+            assert np.array_equal(out[0][f].view(np.uint32), out[1][f].view(np.uint32)), (arithmetic, f)
