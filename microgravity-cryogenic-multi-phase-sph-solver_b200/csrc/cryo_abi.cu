@@ -224,16 +224,16 @@ void cryo_ctx::build_lists(const View& V, int mode) {
 // Solver::evaluate_rates (sph_solver.cu:449-480) on set s.  density_done:
 // the density/EOS pass already ran inside the list build.
 void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool tape) {
-  const int G = grid_blocks();
+  const int G = grid_blocks(), GP = pass_blocks();
   const View V = view(s);
   if (maxima_reset) LAUNCH(k_begin_step, 1, 1, P, V, BEGIN_RATES);
   if (!density_done) {
     if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
-    else FIELD_LAUNCH(k_density, G, kBlock, P, V, 1);
+    else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
     slab_point(SLAB_HALO, s);
   }
   if (rate_lanes(loaded_n - loaded_fluid, WALL_LANES_MAX)) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
-  else FIELD_LAUNCH(k_wall, G, kBlock, P, V);
+  else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
   if (rate_lanes(loaded_fluid, INTERFACE_LANES_MAX)) {
     if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V);
@@ -246,11 +246,11 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
   if (P.thermal && P.heat_power != 0.0f) LAUNCH(k_heat_sum, G, kBlock, P, V, reduce());
   slab_point(P.thermal ? SLAB_HEAT : SLAB_HALO, s);
   if (P.sps) {
-    FIELD_LAUNCH(k_sps, G, kBlock, P, V);
+    FIELD_LAUNCH(k_sps, GP, kBlock, P, V);
     slab_point(SLAB_HALO, s);
   }
   if (P.csf_active && P.csf_smooth) {
-    FIELD_LAUNCH(k_smooth_normals, G, kBlock, P, V);
+    FIELD_LAUNCH(k_smooth_normals, GP, kBlock, P, V);
     slab_point(SLAB_HALO, s);
   }
   const int GF = forces_blocks();
@@ -357,7 +357,7 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   LAUNCH(k_kick, G, kBlock, P, V, (P.cfg_phase_change ? KICK_SOURCES : 0) | KICK_HEAT);
   slab_point(SLAB_HALO, d);
   if (P.shift_strength > 0.0f) {
-    FIELD_LAUNCH(k_shift_compute, G, kBlock, P, V);
+    FIELD_LAUNCH(k_shift_compute, pass_blocks(), kBlock, P, V);
     slab_point(SLAB_HALO, d);
     FIELD_LAUNCH(k_shift_apply, G, kBlock, P, V);
     slab_point(SLAB_HALO, d);
@@ -367,15 +367,15 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
-    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, k_pc_normalize, P, V, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.pc, tape->pc2, nullptr, nullptr, dyn);
-    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, k_pc_apply, P, V, R, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, G, k_pc_apply, P, V, R, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT2, tape->m2, V.mrps, dyn);
     const bool reb = P.vapor_rebalance > 0.0f && has_vapor;
     if (reb) {
-      PASS_LAUNCH(crowded(loaded_fluid) <= PASS_LANES_MAX, k_rebalance1, P, V, 1);
+      PASS_LAUNCH(crowded(loaded_fluid) <= PASS_LANES_MAX, pass_blocks(), k_rebalance1, P, V, 1);
       slab_point(SLAB_HALO, d);
     }
     LAUNCH(k_rebalance2_mark, G, kBlock, P, V, R, split_flag, reb ? 1 : 0, 1);

@@ -52,12 +52,12 @@ struct CudaError : std::runtime_error {
   } while (0)
 
 // A phase-change pass in the shape its size asks for.
-#define PASS_LAUNCH(SMALL, K, ...)                                  \
+#define PASS_LAUNCH(SMALL, BLOCKS, K, ...)                          \
   do {                                                              \
     if (SMALL)                                                      \
       LAUNCH(K<PASS_LANES>, lane_blocks(), kBlock, __VA_ARGS__);    \
     else                                                            \
-      LAUNCH(K<1>, grid_blocks(), kBlock, __VA_ARGS__);             \
+      LAUNCH(K<1>, BLOCKS, kBlock, __VA_ARGS__);                    \
   } while (0)
 
 // A kernel of cryo_physics.cu in the context's field arithmetic (exact: the
@@ -411,6 +411,18 @@ struct cryo_ctx {
     const int need = (span() + per_block - 1) / per_block;
     return std::max(1, std::min(need, sm_count * 8));
   }
+  // A neighbour pass: a thread per particle whatever their number, so that a
+  // block that finds little to do (walls, the other phase) makes room for the
+  // next one.  With a grid of 8 blocks per SM that strides over the particles,
+  // an SM that holds 6 of them ran a second round of 2, and the longest block
+  // set the end: density 855 -> 718 us at 4.08 M particles and 197 -> 169 at
+  // 1.06 M, vapour rebalance 739 -> 692 and 216 -> 199, force pass 4026 -> 3842,
+  // list build 1755 -> 1687.  The phase-change apply pass, which walks whole
+  // chunks, keeps the striding grid (214 us against 234).
+  int pass_blocks() const {
+    const int per_block = kBlock * grid_tile;
+    return std::max(1, (span() + per_block - 1) / per_block);
+  }
   // Which shape a neighbour pass takes depends on the particles loaded, in an
   // ensemble on those that step side by side: lanes pay only while they would
   // otherwise be idle.  Both shapes give the same bits, so a tank steps alike
@@ -427,18 +439,15 @@ struct cryo_ctx {
     const int per_block = INTERFACE_BLOCK * grid_tile;
     return std::max(1, (span() + per_block - 1) / per_block);
   }
-  // force pass: one thread per particle (times the tile) up to two
-  // full-occupancy waves
+  // force pass: one thread per particle (times the tile)
   int forces_blocks() const {
     const int per_block = FORCES_BLOCK * grid_tile;
-    const int need = (span() + per_block - 1) / per_block;
-    return std::max(1, std::min(need, sm_count * (2048 / FORCES_BLOCK) * 2));
+    return std::max(1, (span() + per_block - 1) / per_block);
   }
   // list build, L lanes per particle
   int list_blocks(int L) const {
     const int per_block = kBlock / L * grid_tile;
-    const int need = (span() + per_block - 1) / per_block;
-    return std::max(1, std::min(need, sm_count * 32));
+    return std::max(1, (span() + per_block - 1) / per_block);
   }
   void build_lists(const View& V, int mode);
   void invalidate_graphs() {
