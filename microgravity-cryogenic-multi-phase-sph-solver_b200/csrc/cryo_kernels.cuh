@@ -274,18 +274,18 @@ constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
 #define FORCES_MIN_BLOCKS 9
 #endif
 // The sub-pass sets with surface tension or heat run without spilling at 8
-// blocks per SM (4 warps per sub-partition).  With FORCE_COMMON the fast
-// arithmetic needs fewer registers and takes 10: 778 us against 874 at 1.06 M
-// particles, while the exact one spills there (4235 against 4024 at 4.08 M).
+// blocks per SM (4 warps per sub-partition); the instances with FORCE_COMMON
+// fit 10: 778 us against 874 at 1.06 M particles in the fast arithmetic, 3619
+// against 3842 at 4.08 M in the exact one.  At 12 they spill (963 and 4599 us).
 #ifndef FORCES_MIN_BLOCKS_HEAVY
 #define FORCES_MIN_BLOCKS_HEAVY 8
 #endif
-#ifndef FORCES_MIN_BLOCKS_FAST
-#define FORCES_MIN_BLOCKS_FAST 10
+#ifndef FORCES_MIN_BLOCKS_COMMON
+#define FORCES_MIN_BLOCKS_COMMON 10
 #endif
-constexpr int forces_min_blocks(int what, bool fast) {
+constexpr int forces_min_blocks(int what) {
   return !(what >= 0 && (what & (FORCE_CSF | FORCE_THERMAL))) ? FORCES_MIN_BLOCKS
-         : fast && (what & FORCE_COMMON)                      ? FORCES_MIN_BLOCKS_FAST
+         : what & FORCE_COMMON                                ? FORCES_MIN_BLOCKS_COMMON
                                                               : FORCES_MIN_BLOCKS_HEAVY;
 }
 // Neighbour-loop unroll of the force-pass variants with surface tension or

@@ -389,8 +389,29 @@ __device__ inline float sum_squares(float Vi, float Vi2, float Vj) {
 // over the whole loop: without them 4.08 M particles took 4024 us in place of
 // 4718, 1.06 M in the fast arithmetic 778 in place of 1018, the dam of 204 k
 // 128 in place of 152.
+// A sum of the force pass that few pairs add to (walls, the interface): in
+// registers, or in a column of shared memory that leaves them free over every
+// pair.  With the columns the exact pass of a two-phase tank fits 96 registers
+// and 5 warps per sub-partition instead of 4: 3842 -> 3619 us at 4.08 M
+// particles.  The fast pass fits them anyway and is slower with the columns
+// (771 against 859 us at 1.06 M), and so is the dam's (109 against 113 us).
+template <bool SHARED>
+struct SumV3 {  // in registers
+  V3 v;
+  __device__ SumV3(float*) : v{0, 0, 0} {}
+  __device__ V3 get() const { return v; }
+  __device__ void operator+=(V3 a) { v += a; }
+};
+template <>
+struct SumV3<true> {
+  float* p;
+  __device__ SumV3(float* column) : p(column) { set({0, 0, 0}); }
+  __device__ V3 get() const { return {p[0], p[FORCES_BLOCK], p[2 * FORCES_BLOCK]}; }
+  __device__ void set(V3 v) { p[0] = v.x; p[FORCES_BLOCK] = v.y; p[2 * FORCES_BLOCK] = v.z; }
+  __device__ void operator+=(V3 a) { V3 s = get(); s += a; set(s); }
+};
 template <int WHAT>
-__global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIELD_FAST)) k_forces_t(Params P, View V, int what_rt) {
+__global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_forces_t(Params P, View V, int what_rt) {
   // WHAT >= 0: the sub-pass set is a compile-time constant (the step path);
   // -1: read at run time (operator-level calls)
   const int what = WHAT >= 0 ? WHAT & ~FORCE_COMMON : what_rt;
@@ -413,6 +434,8 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIE
   const bool iso_walls = kCommon ? false : P.wall_bc == CRYO_WALL_ISOTHERMAL;
   const int own_lo = dyn->own_lo, own_hi = dyn->own_hi, n_sorted = dyn->n_sorted;
   float vmax_l = 0.0f, amax_l = 0.0f, tv_l = 0.0f, sr_l = 0.0f, nut_l = 0.0f;
+  constexpr bool kColumns = kCommon && !CRYO_FIELD_FAST && (WHAT & (FORCE_CSF | FORCE_THERMAL));
+  __shared__ float columns[kColumns ? 12 * FORCES_BLOCK : 1];
 
   // walls (and, without lists, every particle that is not fluid): zero outputs
   {
@@ -475,19 +498,20 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIE
     const float VT_i2 = VT_i * VT_i;
     const float mT_i = rhoi * VT_i;
     const float pb = P.tvf_factor * P.rho0[pi_idx] * ci * ci;
-    V3 sumT{0, 0, 0};
+    float* const column = columns + threadIdx.x;
+    SumV3<kColumns> sumT(column);
     // momentum
-    V3 force{0, 0, 0}, acc_av{0, 0, 0}, fwall{0, 0, 0}, mwall{0, 0, 0};
+    V3 force{0, 0, 0}, acc_av{0, 0, 0};
+    SumV3<kColumns> fwall(column + 3 * FORCES_BLOCK), mwall(column + 6 * FORCES_BLOCK);
     const V3 dvi = xyz(vti4) - vi;
     // CSF (surface_tension.cu:131-136)
-    V3 ni{0, 0, 0};
     bool do_C = false;
     if (what & FORCE_CSF) {
-      ni = xyz(V.ns4[i]);
-      do_C = norm2(ni) > 0.25f;
+      do_C = norm2(xyz(V.ns4[i])) > 0.25f;
     }
     const float ciC = ph == kLiquid ? 1.0f : 0.0f;
-    float num = 0.0f, den = 0.0f;
+    SumV3<kColumns> curvature(column + 9 * FORCES_BLOCK);  // {numerator, denominator, -}
+    const V3 ni_held = !kColumns && do_C ? xyz(V.ns4[i]) : V3{0, 0, 0};
     V3 G{0, 0, 0};
     // Akinci
     const bool do_A = (what & FORCE_AKINCI) && ph == kLiquid;
@@ -621,8 +645,8 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIE
         const V3 gwC = separated ? gw : rij * (dW / r);  // the same product where gw is not zeroed
         const V3 nj = xyz(__ldg(V.ns4 + j));
         if (norm2(nj) > 0.25f) {
-          num += Vj * dot(ni - nj, gwC);
-          den += Vj * r * (-dW);
+          const V3 ni = kColumns ? xyz(__ldg(V.ns4 + i)) : ni_held;
+          curvature += V3{Vj * dot(ni - nj, gwC), Vj * r * (-dW), 0.0f};
         }
         if (csf_balanced) {
           const float cj = phj == kLiquid ? 1.0f : 0.0f;
@@ -652,12 +676,12 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIE
     if constexpr (WHAT >= 0 && (WHAT & FORCE_TAPE)) {
       const int tn = V.tape_n;
       V.tape[i] = f4(force, q);
-      V.tape[tn + i] = f4(sumT, num);
-      V.tape[2 * tn + i] = make_float4(den, 0.0f, 0.0f, 0.0f);
+      V.tape[tn + i] = f4(sumT.get(), curvature.get().x);
+      V.tape[2 * tn + i] = make_float4(curvature.get().y, 0.0f, 0.0f, 0.0f);
     }
     V3 ab{0, 0, 0};
     if (what & FORCE_TRANSPORT) {
-      if (do_T) ab = sumT * (-pb / mT_i);
+      if (do_T) ab = sumT.get() * (-pb / mT_i);
       V.ab4[i] = f4(ab, V.ab4[i].w);
     }
     float4 a4 = V.a4[i];
@@ -671,14 +695,15 @@ __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT, CRYO_FIE
         const V3 rr = xi - origin;
         acc -= cross(omega_dot, rr) + cross(omega, cross(omega, rr)) + cross(omega, vi) * 2.0f;
       }
-      V.fw[i] = f4(fwall, 0.0f);
-      V.mw[i] = f4(mwall, 0.0f);
+      V.fw[i] = f4(fwall.get(), 0.0f);
+      V.mw[i] = f4(mwall.get(), 0.0f);
     }
     if (what & FORCE_CSF) {
       float4 ns4 = V.ns4[i];
       if (!do_C) {
         ns4.w = 0.0f;
       } else {
+        const float num = curvature.get().x, den = curvature.get().y;
         const float kappa = den > 0.0f ? 3.0f * num / den : 0.0f;
         ns4.w = kappa;
         if (P.wetting_model != 0) acc += xyz(V.vwp[i]);
