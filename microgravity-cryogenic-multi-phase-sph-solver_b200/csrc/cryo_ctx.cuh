@@ -262,6 +262,8 @@ struct cryo_ctx {
   char* io_dev = nullptr;
   char* io_host = nullptr;
   size_t io_cap = 0;
+  static constexpr int kIoSlices = 16;
+  cudaEvent_t io_ev[kIoSlices] = {};  // slice k of a download has arrived
   void io_reserve(size_t bytes);
 
   // differentiated window (cryo_adj_*), and the sums tape of the step being
@@ -338,6 +340,8 @@ struct cryo_ctx {
     }
     if (ens_ev) cudaEventDestroy(ens_ev);
     telemetry_release();
+    for (cudaEvent_t e : io_ev)
+      if (e) cudaEventDestroy(e);
     if (io_dev || io_host) {
       if (stream) cudaStreamSynchronize(stream);
       if (io_dev) cudaFree(io_dev);
