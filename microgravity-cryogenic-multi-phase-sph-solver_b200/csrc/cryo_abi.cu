@@ -1386,20 +1386,30 @@ int cryo_probe_pressure(cryo_ctx* c, const float* pts, int np, float* out) {
   return guard(c, [&] {
     c->ensure_initialized();
     if (np <= 0) return;
+    // A few points use the context's own scratch, made on the first call: a
+    // pool allocation given back by the synchronisation below cost 0.5 ms a call.
+    const bool kept = np <= cryo_ctx::kProbeKept;
+    std::unique_lock<std::mutex> lock(c->probe_mu, std::defer_lock);
     float* d = nullptr;
-    CK(cudaMallocAsync(&d, (size_t)np * 4 * sizeof(float), c->stream));
+    if (kept) {
+      lock.lock();
+      if (!c->probe_dev) CK(cudaMalloc(&c->probe_dev, cryo_ctx::kProbeKept * 4 * sizeof(float)));
+      d = c->probe_dev;
+    } else {
+      CK(cudaMallocAsync(&d, (size_t)np * 4 * sizeof(float), c->stream));
+    }
     CK(cudaMemcpyAsync(d, pts, (size_t)np * 3 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    const int blocks = std::max(1, std::min((np + 127) / 128, c->sm_count * 8));
-    FIELD_KERNEL(c, k_probe)<<<blocks, 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
+    FIELD_KERNEL(c, k_probe)<<<c->probe_blocks(np), 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
     LAUNCH_CHECK();
     CK(cudaMemcpyAsync(out, d + 3 * (size_t)np, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaFreeAsync(d, c->stream));
+    if (!kept) CK(cudaFreeAsync(d, c->stream));
     c->sync();
   });
 }
 
 // Solver::probe_pressure without device allocation. cryo_probe_pressure
-// takes its point/result buffer from the stream-ordered pool on every call;
+// makes its scratch on the first call, or takes a buffer for many points from
+// the stream-ordered pool on every call;
 // this variant stages through one fixed array per device instead. It is for
 // callers that must not allocate device memory once running: a monitoring or
 // control loop that probes tank pressure every cycle under a fixed memory
@@ -1452,8 +1462,7 @@ int cryo_probe_pressure_noalloc(cryo_ctx* c, const float* pts, int np, float* ou
       d = static_cast<float*>(p);
     }
     CK(cudaMemcpyAsync(d, pts, (size_t)np * 3 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    const int blocks = std::max(1, std::min((np + 127) / 128, c->sm_count * 8));
-    FIELD_KERNEL(c, k_probe)<<<blocks, 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
+    FIELD_KERNEL(c, k_probe)<<<c->probe_blocks(np), 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
     LAUNCH_CHECK();
     CK(cudaMemcpyAsync(out, d + 3 * (size_t)np, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     c->sync();

@@ -266,6 +266,13 @@ struct cryo_ctx {
   cudaEvent_t io_ev[kIoSlices] = {};  // slice k of a download has arrived
   void io_reserve(size_t bytes);
 
+  // scratch of probe_pressure: up to kProbeKept points and their results, made
+  // on the first call
+  static constexpr int kProbeKept = 1024;
+  float* probe_dev = nullptr;
+  std::mutex probe_mu;
+  int probe_blocks(int np) const { return std::max(1, std::min((np + 3) / 4, sm_count * 16)); }
+
   // differentiated window (cryo_adj_*), and the sums tape of the step being
   // recomputed for it (View::tape; null otherwise)
   AdjWindow* adj = nullptr;
@@ -340,6 +347,10 @@ struct cryo_ctx {
     }
     if (ens_ev) cudaEventDestroy(ens_ev);
     telemetry_release();
+    if (probe_dev) {
+      if (stream) cudaStreamSynchronize(stream);
+      cudaFree(probe_dev);
+    }
     for (cudaEvent_t e : io_ev)
       if (e) cudaEventDestroy(e);
     if (io_dev || io_host) {

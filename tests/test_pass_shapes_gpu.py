@@ -207,3 +207,24 @@ def test_force_pass_without_the_rarer_options(cuda_device, base, other, arithmet
             out.append({f: g.field(f) for f in ("x", "v", "rho", "T", "a", "ab", "drho", "dTdt", "fw", "mw")})
         for f in out[0]:
             assert np.array_equal(out[0][f].view(np.uint32), out[1][f].view(np.uint32)), (arithmetic, f)
+
+
+@pytest.mark.parametrize("np_", [1, 3, 4, 5, 1024, 1025])
+def test_probes_by_warps(cuda_device, np_):
+    """Any number of points gives each point's own value, that of the sum over
+    the liquid (a term is within 16 ulp, at most ~100 of them are added)."""
+    cfg = free_surface_config(0.02)
+    g = cabi.Context(cfg, cabi.py_fluid(cabi.FLUID_H2O))
+    g.set_particles(cloud(6000, 11), LO, HI)
+    g.step(1)
+    pts = np.random.default_rng(np_).uniform((-0.05, -0.05, -0.05), (0.45, 0.35, 0.25), (np_, 3)).astype(np.float32)
+    p = np.asarray(g.probe_pressure(pts))
+    for k in range(0, np_, max(1, np_ // 5)):
+        one = np.asarray(g.probe_pressure(pts[k:k + 1]))
+        assert np.array_equal(one.view(np.uint32), p[k:k + 1].view(np.uint32)) or (np.isnan(one[0]) and np.isnan(p[k]))
+        h = 0.02 * 1.3
+        q = np.linalg.norm(g.field("x").astype(np.float64) - pts[k].astype(np.float64), axis=1) / h
+        w = np.where(q < 2, (1 - q / 2) ** 4 * (2 * q + 1), 0.0) * g.field("m") / g.field("rho")
+        if w.sum() > 1e-3 * (1e-3 / 1000):
+            term = w * g.field("p")
+            assert abs(one[0] - term.sum() / w.sum()) <= 2e-4 * np.abs(term).sum() / w.sum()
