@@ -236,11 +236,11 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool 
   else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
   if (rate_lanes(loaded_fluid, INTERFACE_LANES_MAX)) {
-    if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V);
-    else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V);
+    if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, 1);
+    else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, 1);
   } else {
-    if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V);
-    else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V);
+    if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V, 1);
+    else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V, 1);
   }
   // without a heater there is nothing to normalise: the force pass reads a zero power
   if (P.thermal && P.heat_power != 0.0f) LAUNCH(k_heat_sum, G, kBlock, P, V, reduce());
@@ -1514,7 +1514,7 @@ int cryo_pass(cryo_ctx* c, int pass) {
       case CRYO_PASS_NORMALIZE_MASSES: FIELD_KERNEL(c, k_normalize_masses)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_EOS: FIELD_KERNEL(c, k_eos)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_WALL_BOUNDARY: FIELD_KERNEL(c, k_wall)<<<G, kBlock, 0, st>>>(P, V); break;
-      case CRYO_PASS_INTERFACE: FIELD_KERNEL(c, k_interface<0>)<<<c->interface_blocks(), INTERFACE_BLOCK, 0, st>>>(P, V); break;
+      case CRYO_PASS_INTERFACE: FIELD_KERNEL(c, k_interface<0>)<<<c->interface_blocks(), INTERFACE_BLOCK, 0, st>>>(P, V, 0); break;
       case CRYO_PASS_TRANSPORT: FIELD_KERNEL(c, k_forces_t<-1>)<<<c->forces_blocks(), FORCES_BLOCK, 0, st>>>(P, V, FORCE_TRANSPORT); break;
       case CRYO_PASS_SPS: FIELD_KERNEL(c, k_sps)<<<G, kBlock, 0, st>>>(P, V); break;
       case CRYO_PASS_MOMENTUM: FIELD_KERNEL(c, k_forces_t<-1>)<<<c->forces_blocks(), FORCES_BLOCK, 0, st>>>(P, V, FORCE_MOMENTUM); break;

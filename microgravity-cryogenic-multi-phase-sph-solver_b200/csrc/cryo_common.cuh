@@ -232,7 +232,8 @@ struct View {
   uint32_t* cell_kinds;
   // lists mode, per particle: the kinds of all cells its neighbours can be in
   // (set by the list build; a particle with no wall and none of the other
-  // phase around skips the interface pass)
+  // phase around skips the interface pass of a step.  They describe the sorted
+  // particles: a phase set or a position shifted since does not show here)
   uint8_t* near_kinds;
   DynState* dyn;
   // maneuver table

@@ -233,7 +233,7 @@ enum { FORCE_TRANSPORT = 1, FORCE_MOMENTUM = 2, FORCE_CSF = 4, FORCE_AKINCI = 8,
   __global__ void k_eos(Params P, View V);                                          \
   __global__ void k_wall(Params P, View V);                                         \
   template <int TAPE>                                                               \
-  __global__ void k_interface(Params P, View V);                                    \
+  __global__ void k_interface(Params P, View V, int sorted);                        \
   __global__ void k_sps(Params P, View V);                                          \
   __global__ void k_smooth_normals(Params P, View V);                               \
   template <int WHAT>                                                               \
@@ -253,7 +253,7 @@ namespace lanes {
 __global__ void k_density(Params P, View V);
 __global__ void k_wall(Params P, View V);
 template <int TAPE>
-__global__ void k_interface(Params P, View V);
+__global__ void k_interface(Params P, View V, int sorted);
 template <int WHAT>
 __global__ void k_forces_t(Params P, View V);
 }

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kBlock) k_wall(Params P, View V) {
 
 // compute_interface_fields (surface_tension.cu:5-85), as exact::k_interface.
 template <int TAPE>
-__global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V) {
+__global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V, int sorted) {
   const Range rg = fluid_range(P, V);
   const bool write_ns = P.csf_active && !P.csf_smooth;
   const int sub = threadIdx.x % L;
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V)
     // as in exact::k_interface: only walls count in a tank without vapour
     const bool walls_only = !TAPE && !P.has_vapor && P.st_model != CRYO_ST_AKINCI;
     // (and a particle with no wall and none of the other phase around it has only zeros to add)
-    const bool alone = !TAPE && P.st_model != CRYO_ST_AKINCI &&
+    const bool alone = !TAPE && sorted && P.st_model != CRYO_ST_AKINCI &&
                        !(V.near_kinds[i] & (kNearWall | (ph == kVapor ? kNearLiquid : kNearVapor)));
     NbrRounds<L> nbrs(P, V, i, xi, sub, live && !alone);
     // the sums a round has no term for are left alone
@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V)
     }
   }
 }
-template __global__ void k_interface<0>(Params, View);
-template __global__ void k_interface<1>(Params, View);
+template __global__ void k_interface<0>(Params, View, int);
+template __global__ void k_interface<1>(Params, View, int);
 
 // The fused force pass of exact::k_forces_t (cryo_physics.cu: what it covers
 // and why it may be fused).  The pairs' terms go through shared memory, one row

@@ -161,8 +161,10 @@ __global__ void __launch_bounds__(kBlock) k_wall(Params P, View V) {
 // walk their lists and the others do not, so the blocks are small, none waits
 // for its other warps, and there is one per INTERFACE_BLOCK particles: the
 // warps that finish at once make room for others.
+// sorted: positions and phases are those the lists were built from, hence
+// near_kinds holds.  An operator call (0) takes the phases as they are now.
 template <int TAPE>
-__global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V) {
+__global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V, int sorted) {
   const Range rg = fluid_range(P, V);
   const bool write_ns = P.csf_active && !P.csf_smooth;
   {
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V)
       // around it: s_other is 0, so alpha is 0 whatever s_all is, and every
       // other sum stays empty.  Away from walls and interfaces (four fifths of
       // a 4 M-particle sphere) the pass then walks no list.
-      if (!TAPE && P.use_lists && P.st_model != CRYO_ST_AKINCI && is_fluid(ph) &&
+      if (!TAPE && sorted && P.use_lists && P.st_model != CRYO_ST_AKINCI && is_fluid(ph) &&
           !(V.near_kinds[i] & (kNearWall | (ph == kVapor ? kNearLiquid : kNearVapor)))) {
         V.wall_w[i] = 0.0f;
         V.heat_w[i] = 0.0f;
@@ -280,8 +282,8 @@ __global__ void __launch_bounds__(INTERFACE_BLOCK) k_interface(Params P, View V)
   }
 }
 
-template __global__ void k_interface<0>(Params, View);
-template __global__ void k_interface<1>(Params, View);
+template __global__ void k_interface<0>(Params, View, int);
+template __global__ void k_interface<1>(Params, View, int);
 
 // compute_sps_viscosity (navier_stokes.cu:71-119)
 __global__ void __launch_bounds__(kBlock) k_sps(Params P, View V) {
