@@ -221,26 +221,24 @@ void cryo_ctx::build_lists(const View& V, int mode) {
     LAUNCH(k_build_lists<1>, list_blocks(1), kBlock, P, V, reduce(), mode);
 }
 
-// Solver::evaluate_rates (sph_solver.cu:449-480) on set s.  density_done:
-// the density/EOS pass already ran inside the list build.
-void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool density_done, bool tape) {
+// Solver::evaluate_rates (sph_solver.cu:449-480) on set s.  sorted: the sort
+// ran just before, so what it noted of the cells (View::near_kinds) holds.
+void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) {
   const int G = grid_blocks(), GP = pass_blocks();
   const View V = view(s);
   if (maxima_reset) LAUNCH(k_begin_step, 1, 1, P, V, BEGIN_RATES);
-  if (!density_done) {
-    if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
-    else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
-    slab_point(SLAB_HALO, s);
-  }
+  if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
+  else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
+  slab_point(SLAB_HALO, s);
   if (rate_lanes(loaded_n - loaded_fluid, WALL_LANES_MAX)) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
   if (rate_lanes(loaded_fluid, INTERFACE_LANES_MAX)) {
-    if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, 1);
-    else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, 1);
+    if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
+    else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
   } else {
-    if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V, 1);
-    else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V, 1);
+    if (tape) FIELD_LAUNCH(k_interface<1>, interface_blocks(), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
+    else FIELD_LAUNCH(k_interface<0>, interface_blocks(), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
   }
   // without a heater there is nothing to normalise: the force pass reads a zero power
   if (P.thermal && P.heat_power != 0.0f) LAUNCH(k_heat_sum, G, kBlock, P, V, reduce());
@@ -343,7 +341,7 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   const int d = 1 - s;
   const View V = view(d);
   slab_point(SLAB_SORTED, d);
-  evaluate_rates(d, false, false, tape != nullptr);
+  evaluate_rates(d, false, true, tape != nullptr);
   if (tape) {
     LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT1, tape->m1, V.mrps, dyn);
     LAUNCH(k_adj_copy4, G, kBlock, V.ns4, tape->ns1, nullptr, nullptr, dyn);
@@ -442,7 +440,7 @@ void cryo_ctx::ensure_initialized() {
     FIELD_LAUNCH(k_normalize_masses, G, kBlock, P, view(cur));
     slab_point(SLAB_HALO, cur);
   }
-  evaluate_rates(cur, true, false);
+  evaluate_rates(cur, true, true);
   LAUNCH(k_saturation, G, kBlock, P, view(cur), reduce(), 0);
   slab_point(SLAB_END, cur);
   initialized = true;

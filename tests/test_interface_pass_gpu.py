@@ -58,3 +58,22 @@ def test_interface_pass_takes_the_phases_as_they_are(cuda_device, arithmetic):
         g.run_pass("interface")
         out.append({f: g.field(f) for f in FIELDS})
     same(*out)
+
+
+@pytest.mark.parametrize("arithmetic", [0, 1])
+def test_rates_after_relax_take_the_phases_as_they_are(cuda_device, arithmetic):
+    """relax() closes with an evaluation of the rates that no sort precedes:
+    it leaves the interface fields an operator pass gives, and in the exact
+    arithmetic the rates found without lists."""
+    out = []
+    for lists in (1, 0):
+        g = tank(arithmetic, lists)
+        g.step(1)
+        turn_a_blob_over(g)
+        g.relax(0.0)
+        out.append({f: g.field(f) for f in FIELDS + ("a", "kappa", "p")})
+        left = {f: g.field(f) for f in FIELDS}
+        g.run_pass("interface")
+        same(left, {f: g.field(f) for f in FIELDS})
+    if arithmetic == 0:
+        same(*out)
