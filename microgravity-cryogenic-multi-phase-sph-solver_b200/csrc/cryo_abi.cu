@@ -1379,6 +1379,24 @@ int cryo_damp_velocities(cryo_ctx* c, float factor) {
   });
 }
 
+}  // extern "C"
+
+// The probe in the shape its count asks for.
+void cryo_ctx::probe(const float* points, int np, float* out) {
+  constexpr int kThreads = 128;
+  const View V = view(cur);
+  if (np <= PROBE_WARPS_MAX) {
+    const int G = std::max(1, std::min((np + kThreads / 32 - 1) / (kThreads / 32), sm_count * 16));
+    FIELD_KERNEL(this, k_probe<32>)<<<G, kThreads, 0, stream>>>(P, V, points, np, out);
+  } else {
+    const int G = std::max(1, std::min((np + kThreads - 1) / kThreads, sm_count * 16));
+    FIELD_KERNEL(this, k_probe<1>)<<<G, kThreads, 0, stream>>>(P, V, points, np, out);
+  }
+  LAUNCH_CHECK();
+}
+
+extern "C" {
+
 // Solver::probe_pressure (sph_solver.cu:738-748)
 int cryo_probe_pressure(cryo_ctx* c, const float* pts, int np, float* out) {
   return guard(c, [&] {
@@ -1397,8 +1415,7 @@ int cryo_probe_pressure(cryo_ctx* c, const float* pts, int np, float* out) {
       CK(cudaMallocAsync(&d, (size_t)np * 4 * sizeof(float), c->stream));
     }
     CK(cudaMemcpyAsync(d, pts, (size_t)np * 3 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    FIELD_KERNEL(c, k_probe)<<<c->probe_blocks(np), 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
-    LAUNCH_CHECK();
+    c->probe(d, np, d + 3 * (size_t)np);
     CK(cudaMemcpyAsync(out, d + 3 * (size_t)np, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     if (!kept) CK(cudaFreeAsync(d, c->stream));
     c->sync();
@@ -1460,8 +1477,7 @@ int cryo_probe_pressure_noalloc(cryo_ctx* c, const float* pts, int np, float* ou
       d = static_cast<float*>(p);
     }
     CK(cudaMemcpyAsync(d, pts, (size_t)np * 3 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    FIELD_KERNEL(c, k_probe)<<<c->probe_blocks(np), 128, 0, c->stream>>>(c->P, c->view(c->cur), d, np, d + 3 * (size_t)np);
-    LAUNCH_CHECK();
+    c->probe(d, np, d + 3 * (size_t)np);
     CK(cudaMemcpyAsync(out, d + 3 * (size_t)np, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     c->sync();
   });

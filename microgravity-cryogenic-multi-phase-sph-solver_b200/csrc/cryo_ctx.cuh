@@ -271,7 +271,7 @@ struct cryo_ctx {
   static constexpr int kProbeKept = 1024;
   float* probe_dev = nullptr;
   std::mutex probe_mu;
-  int probe_blocks(int np) const { return std::max(1, std::min((np + 3) / 4, sm_count * 16)); }
+  void probe(const float* points, int np, float* out);
 
   // differentiated window (cryo_adj_*), and the sums tape of the step being
   // recomputed for it (View::tape; null otherwise)

@@ -241,6 +241,7 @@ enum { FORCE_TRANSPORT = 1, FORCE_MOMENTUM = 2, FORCE_CSF = 4, FORCE_AKINCI = 8,
   __global__ void k_maxima(Params P, View V);                                       \
   __global__ void k_shift_compute(Params P, View V);                                \
   __global__ void k_shift_apply(Params P, View V);                                  \
+  template <int LANES>                                                              \
   __global__ void k_probe(Params P, View V, const float* pts, int np, float* out);
 namespace exact {
 CRYO_FIELD_KERNELS
@@ -330,6 +331,17 @@ constexpr int FORCES_LANED_BLOCK = 128;
 #endif
 #ifndef WALL_LANES_MAX
 #define WALL_LANES_MAX 60000
+#endif
+
+// Points a pressure probe gives a warp each; more take a thread each.  A warp
+// shortens a point's chain but adds its ~75 terms one after another for 32
+// lanes.  Kernel, us, warps against threads (27 k / 204 k / 840 k particles):
+//   random points, 1 024    17 / 17 / 17      against  206 / 266 / 269
+//   a lattice,    32 768    80 / 94 / 97               102 / 126 / 209
+//   a lattice,    64 000   150 / 168 / 181             110 / 157 / 226
+//   a lattice, 1 061 208  2249 / 2682 / 2802           659 / 959 / 1188
+#ifndef PROBE_WARPS_MAX
+#define PROBE_WARPS_MAX 32768
 #endif
 
 // integrator + phase change (cryo_phase.cu)

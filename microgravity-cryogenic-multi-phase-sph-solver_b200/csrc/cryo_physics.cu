@@ -879,46 +879,67 @@ __global__ void __launch_bounds__(kBlock) k_shift_apply(Params P, View V) {
 // adds the accepted ones in the order of the scan, so few points (a tank has a
 // handful of sensors) are a chain of ~20 loads instead of ~470.  With the
 // context's own scratch a call for eight points takes 32 us in place of 580.
-__global__ void __launch_bounds__(128) k_probe(Params P, View V, const float* __restrict__ pts, int np,
-                                               float* __restrict__ out) {
+__device__ inline float probe_by_warp(const Params& P, const View& V, V3 x) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / 32; k < np; k += gridDim.x * blockDim.x / 32) {
-    const V3 x = v3(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]);
-    float num = 0.0f, den = 0.0f;
-    const CellWindow W(P, x);
-    for (int z = W.z0; z <= W.z1; ++z) {
-      for (int y = W.y0; y <= W.y1; ++y) {
-        int xs, xe;
-        if (!W.row(P, y, z, xs, xe)) continue;
-        const int row = (z * P.ny + y) * P.nx;
-        const int e = __ldg(V.cell_begin + row + xe + 1);
-        for (int j0 = __ldg(V.cell_begin + row + xs); j0 < e; j0 += 32) {
-          const int j = j0 + lane;
-          bool in = false;
-          float w = 0.0f, p = 0.0f;
-          if (j < e) {
-            const float4 xj = __ldg(V.xp + j);
-            const float r2 = norm2(x - xyz(xj));
-            if (!(r2 >= P.support2) && ph_of(xj) == kLiquid) {
-              const float4 mr = __ldg(V.mrps + j);
-              in = true;
-              w = (mr.x / mr.y) * kernel_W(P, sqrtf(r2));
-              p = mr.z;
-            }
+  float num = 0.0f, den = 0.0f;
+  const CellWindow W(P, x);
+  for (int z = W.z0; z <= W.z1; ++z) {
+    for (int y = W.y0; y <= W.y1; ++y) {
+      int xs, xe;
+      if (!W.row(P, y, z, xs, xe)) continue;
+      const int row = (z * P.ny + y) * P.nx;
+      const int e = __ldg(V.cell_begin + row + xe + 1);
+      for (int j0 = __ldg(V.cell_begin + row + xs); j0 < e; j0 += 32) {
+        const int j = j0 + lane;
+        bool in = false;
+        float w = 0.0f, p = 0.0f;
+        if (j < e) {
+          const float4 xj = __ldg(V.xp + j);
+          const float r2 = norm2(x - xyz(xj));
+          if (!(r2 >= P.support2) && ph_of(xj) == kLiquid) {
+            const float4 mr = __ldg(V.mrps + j);
+            in = true;
+            w = (mr.x / mr.y) * kernel_W(P, sqrtf(r2));
+            p = mr.z;
           }
-          for (unsigned m = __ballot_sync(kAll, in); m; m &= m - 1) {
-            const int b = __ffs(m) - 1;
-            const float wb = __shfl_sync(kAll, w, b);
-            num += __shfl_sync(kAll, p, b) * wb;
-            den += wb;
-          }
+        }
+        for (unsigned m = __ballot_sync(kAll, in); m; m &= m - 1) {
+          const int b = __ffs(m) - 1;
+          const float wb = __shfl_sync(kAll, w, b);
+          num += __shfl_sync(kAll, p, b) * wb;
+          den += wb;
         }
       }
     }
-    if (lane == 0) out[k] = den > 0.0f ? num / den : __int_as_float(0x7fc00000);
+  }
+  return den > 0.0f ? num / den : __int_as_float(0x7fc00000);
+}
+// LANES 32: a warp per point; 1: a thread per point, for more points than
+// PROBE_WARPS_MAX.  Both add the same terms in the same order.
+template <int LANES>
+__global__ void __launch_bounds__(128) k_probe(Params P, View V, const float* pts, int np, float* out) {
+  const int step = gridDim.x * (blockDim.x / LANES);
+  for (int k = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; k < np; k += step) {
+    const V3 x = v3(pts[3 * k], pts[3 * k + 1], pts[3 * k + 2]);
+    if constexpr (LANES == 32) {
+      const float p = probe_by_warp(P, V, x);
+      if ((threadIdx.x & 31) == 0) out[k] = p;
+    } else {
+      float num = 0.0f, den = 0.0f;
+      for_each_neighbor(P, V.cell_begin, V.xp, x, [&](int j, float4 xj, V3, float r2) {
+        if (ph_of(xj) != kLiquid) return;
+        const float4 mr = __ldg(V.mrps + j);
+        const float w = (mr.x / mr.y) * kernel_W(P, sqrtf(r2));
+        num += mr.z * w;
+        den += w;
+      });
+      out[k] = den > 0.0f ? num / den : __int_as_float(0x7fc00000);
+    }
   }
 }
+template __global__ void k_probe<1>(Params, View, const float*, int, float*);
+template __global__ void k_probe<32>(Params, View, const float*, int, float*);
 
 }  // namespace CRYO_FIELD_NS
 }  // namespace cryo

@@ -228,3 +228,18 @@ def test_probes_by_warps(cuda_device, np_):
         if w.sum() > 1e-3 * (1e-3 / 1000):
             term = w * g.field("p")
             assert abs(one[0] - term.sum() / w.sum()) <= 2e-4 * np.abs(term).sum() / w.sum()
+
+
+@pytest.mark.parametrize("arithmetic", [0, 1])
+@pytest.mark.parametrize("np_", [32768, 32769, 40001])
+def test_probes_of_many_points(cuda_device, np_, arithmetic):
+    """Above 32 768 points each has a thread instead of a warp: the same bits."""
+    g = cabi.Context(free_surface_config(0.02), cabi.py_fluid(cabi.FLUID_H2O))
+    g.set_field_arithmetic(arithmetic)
+    g.set_particles(cloud(6000, 11), LO, HI)
+    g.step(1)
+    pts = np.random.default_rng(np_).uniform((-0.05, -0.05, -0.05), (0.45, 0.35, 0.25), (np_, 3)).astype(np.float32)
+    p = np.asarray(g.probe_pressure(pts))
+    parts = np.concatenate([np.asarray(g.probe_pressure(q)) for q in np.array_split(pts, 9)])
+    assert np.array_equal(np.isnan(p), np.isnan(parts)) and 0 < np.isnan(p).sum() < np_
+    assert np.array_equal(p[~np.isnan(p)].view(np.uint32), parts[~np.isnan(p)].view(np.uint32))
