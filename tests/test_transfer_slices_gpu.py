@@ -34,3 +34,26 @@ def test_round_trip(cuda_device, n, optional, dtype):
     if optional:
         for k in ("velocity", "normal", "flags"):
             assert np.array_equal(q[k][order], extra[k].astype(q[k].dtype)), k
+
+
+@pytest.mark.parametrize("n", [35_000, 36_500, 50_000, 72_000])
+def test_one_slice_of_doubles(cuda_device, n):
+    """Below one slice, doubles of more than 4 MiB are copied by several threads."""
+    test_round_trip(cuda_device, n, True, np.float64)
+
+
+@pytest.mark.parametrize("n", [1, 15, 17, 4099])
+def test_phases_are_counted(cuda_device, n):
+    """A tank is two-phase if any of its particles, the last included, is vapour."""
+    cfg = cs.SolverConfig()
+    cfg.dx = 0.01
+    cfg.surface_tension = cs.SurfaceTensionModel.Akinci
+    x = np.random.default_rng(n).uniform(0, 1, (n, 3))
+    full = np.full(n, 1.0)
+    for k in sorted({0, n // 2, n - 1}):
+        phase = np.full(n, 2, np.uint8)
+        s = cs.Solver(cfg, cs.FluidProperties.water())
+        s.set_particles(x, full, full, full, phase, domain_lo=(0, 0, 0), domain_hi=(1, 1, 1))
+        phase[k] = 1  # Akinci's model takes no vapour
+        with pytest.raises(ValueError):
+            s.set_particles(x, full, full, full, phase, domain_lo=(0, 0, 0), domain_hi=(1, 1, 1))
