@@ -230,10 +230,14 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
   if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
   slab_point(SLAB_HALO, s);
-  if (rate_lanes(loaded_n - loaded_fluid, WALL_LANES_MAX)) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
+  if (rate_lanes(loaded_n - loaded_fluid, P.has_vapor ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID))
+    LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
-  if (rate_lanes(loaded_fluid, INTERFACE_LANES_MAX)) {
+  const int interface_max = P.st_model == CRYO_ST_AKINCI ? INTERFACE_LANES_MAX_AKINCI
+                            : P.has_vapor                ? INTERFACE_LANES_MAX
+                                                         : INTERFACE_LANES_MAX_WALLS;
+  if (rate_lanes(loaded_fluid, interface_max)) {
     if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
     else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
   } else {
@@ -365,10 +369,10 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
-    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= PC_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.pc, tape->pc2, nullptr, nullptr, dyn);
-    PASS_LAUNCH(crowded(loaded_fluid) <= INTERFACE_LANES_MAX, G, k_pc_apply, P, V, R, 1);
+    PASS_LAUNCH(crowded(loaded_fluid) <= PC_LANES_MAX, G, k_pc_apply, P, V, R, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT2, tape->m2, V.mrps, dyn);
     const bool reb = P.vapor_rebalance > 0.0f && has_vapor;

@@ -296,8 +296,9 @@ constexpr int forces_min_blocks(int what) {
 #define FORCES_UNROLL_HEAVY 2
 #endif
 // Neighbour-list build: LIST_LANES lanes per particle up to LIST_LANES_MAX
-// particles, one above (k_build_lists): lanes 25 us against 41 at 27 k, 81
-// against 68 at 91 k, 93 against 78 at 204 k.
+// particles, one above (k_build_lists).  One thread against lanes, us: 42 / 39
+// at 37 k particles, 52 / 57 at 55 k, 50 / 47 at 60 k (free surface, twice the
+// walls), 60 / 74 at 85 k.
 constexpr int LIST_LANES = 4;
 constexpr int kListPad = 8;  // records the build may load beyond the last particle
 #ifndef LIST_LANES_MAX
@@ -308,29 +309,52 @@ constexpr int kListPad = 8;  // records the build may load beyond the last parti
 // particles; walls for the wall pass; in an ensemble those of the tanks that
 // step side by side).  Lanes shorten the chain of a particle's ~75 neighbours
 // but add shuffles and rows, so they pay while the chip has room for the
-// threads.  Measured one thread against lanes, us per launch (event overhead
-// of ~5 us included):
-//   fluid particles        1 000      14 500     61 000     82 350
-//   force pass, exact    158 / 36   159 / 58       -       153 / 190
-//   density               29 / 15    32 / 19    31 / 45    35 / 52
-//   interface             77 / 22    78 / 28    68 / 42    62 / 44
-//   phase-change apply    31 / 18    39 / 21    44 / 30
-//   vapour rebalance      33 / 17    36 / 21    37 / 39
-// and the wall pass 21 / 15 at 12 000 walls, 23 / 15 at 30 000, 23 / 27 at
-// 121 000.
+// threads.  One thread against lanes, us per launch in the exact arithmetic
+// (event overhead of ~5 us included), boxes at 4 mm:
+//   fluid particles       1 000   13 800   32 800    54 900    74 100   97 300  125 000  157 500
+//   force pass, 2 phases 148/37   149/58  163/101   174/153   187/196  199/249  217/316  253/395
+//   density               27/15    31/20    33/32     35/44     35/55    40/71    42/86   50/110
+//   vapour rebalance      33/17    37/21    40/31     41/43     42/49    44/63    56/74    59/94
+//   interface, 2 phases   69/21    70/27    76/42     81/54     84/67    87/75    89/96   90/100
+//   ph.-change normalize  29/13    29/14    42/17     42/17     42/20    43/21    44/21    34/21
+//   phase-change apply    37/18    39/19    50/27     50/29     51/35    51/44    52/48    47/56
+//   fluid, free surface   2 300    18 400   30 300    55 000    70 000   87 700  107 800  161 200
+//   force pass           117/31    131/59   142/95   165/150   184/189  194/236  271/285  318/427
+//   force pass, Akinci        -    262/84  273/117   291/185   301/226  331/278  439/325        -
+//   interface             54/18     56/24    58/27     58/36     61/42    61/46    66/50    68/64
+//   interface, Akinci         -     78/41    80/55     84/83    89/102   94/124   98/145        -
+//   walls                 2 900    12 800   22 100    30 300    35 600   42 600   49 900   57 800
+//   wall pass, 2 phases   19/13     21/13    21/19     21/21     21/23    23/27    22/29    23/33
+//   wall pass, 1 phase        -     20/13    21/13     21/15     21/17    21/19    21/21    23/23
+// The interface pass crosses late where only walls count (no vapour), early in
+// Akinci's model, which sums over every neighbour.  The force pass's line is
+// the step's: with lanes 280 -> 275 us at 48 400 fluid particles (free surface),
+// 419 -> 380 at 46 700 (two phases), but 288 -> 299 at 55 000 (free surface).
 constexpr int PASS_LANES = 8;
 constexpr int FORCES_LANED_BLOCK = 128;
 #ifndef FORCES_LANES_MAX
-#define FORCES_LANES_MAX 45000
+#define FORCES_LANES_MAX 50000
 #endif
-#ifndef PASS_LANES_MAX
+#ifndef PASS_LANES_MAX  // density, vapour rebalance
 #define PASS_LANES_MAX 40000
 #endif
+#ifndef PC_LANES_MAX  // phase-change normalize and apply
+#define PC_LANES_MAX 130000
+#endif
 #ifndef INTERFACE_LANES_MAX
-#define INTERFACE_LANES_MAX 130000
+#define INTERFACE_LANES_MAX 110000
+#endif
+#ifndef INTERFACE_LANES_MAX_WALLS  // no vapour: walls only
+#define INTERFACE_LANES_MAX_WALLS 130000
+#endif
+#ifndef INTERFACE_LANES_MAX_AKINCI
+#define INTERFACE_LANES_MAX_AKINCI 55000
 #endif
 #ifndef WALL_LANES_MAX
-#define WALL_LANES_MAX 60000
+#define WALL_LANES_MAX 30000
+#endif
+#ifndef WALL_LANES_MAX_LIQUID  // no vapour
+#define WALL_LANES_MAX_LIQUID 57000
 #endif
 
 // Points a pressure probe gives a warp each; more take a thread each.  A warp

@@ -278,7 +278,7 @@ template __global__ void k_interface<1>(Params, View, int);
 // thread of the one-thread pass holds 25, and the eight additions per round are
 // spread over the lanes.  Measured: 159 -> 58 us on the heated 26k-particle
 // cylinder, 158 -> 36 us on a 4k-particle box, 124 -> 29 us on a 27k-particle
-// dam break; at 82k fluid particles it is slower (190 against 153 us: a pair
+// dam break; at 97k fluid particles it is slower (249 against 199 us: a pair
 // costs 1.75 times the instructions), hence FORCES_LANES_MAX.
 enum {  // rows
   kRowP = 0, kRowC = 3, kRowA = 6, kRowX = 9, kRowF = 12, kRowA1 = 15, kRowA2 = 18, kRowS = 21, kRowT = 24,
