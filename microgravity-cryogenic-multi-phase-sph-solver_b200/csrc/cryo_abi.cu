@@ -215,7 +215,7 @@ void cryo_ctx::sort_and_gather(int src, int list_mode, bool reset_maxima) {
 }
 
 void cryo_ctx::build_lists(const View& V, int mode) {
-  if (crowded(loaded_n) <= LIST_LANES_MAX)
+  if (list_lanes())
     LAUNCH(k_build_lists<LIST_LANES>, list_blocks(LIST_LANES), kBlock, P, V, reduce(), mode);
   else
     LAUNCH(k_build_lists<1>, list_blocks(1), kBlock, P, V, reduce(), mode);
@@ -227,17 +227,16 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
   const int G = grid_blocks(), GP = pass_blocks();
   const View V = view(s);
   if (maxima_reset) LAUNCH(k_begin_step, 1, 1, P, V, BEGIN_RATES);
-  if (rate_lanes(loaded_fluid, PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
+  if (rate_lanes(fluid_beside(), PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
   slab_point(SLAB_HALO, s);
-  if (rate_lanes(loaded_n - loaded_fluid, P.has_vapor ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID))
-    LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
+  if (wall_lanes()) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
   const int interface_max = P.st_model == CRYO_ST_AKINCI ? INTERFACE_LANES_MAX_AKINCI
                             : P.has_vapor                ? INTERFACE_LANES_MAX
                                                          : INTERFACE_LANES_MAX_WALLS;
-  if (rate_lanes(loaded_fluid, interface_max)) {
+  if (rate_lanes(fluid_beside(), interface_max)) {
     if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
     else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
   } else {
@@ -256,7 +255,7 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
     slab_point(SLAB_HALO, s);
   }
   const int GF = forces_blocks();
-  const bool laned = rate_lanes(loaded_fluid, FORCES_LANES_MAX);
+  const bool laned = rate_lanes(fluid_beside(), FORCES_LANES_MAX);
   const int GL = lane_blocks(FORCES_LANED_BLOCK);
   // The instances with the rarer options compiled out (cryo_physics.cu).  In
   // the fast arithmetic only four sets have one: those where every sum is known
@@ -369,15 +368,15 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
-    PASS_LAUNCH(crowded(loaded_fluid) <= PC_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
+    PASS_LAUNCH(fluid_beside() <= PC_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.pc, tape->pc2, nullptr, nullptr, dyn);
-    PASS_LAUNCH(crowded(loaded_fluid) <= PC_LANES_MAX, G, k_pc_apply, P, V, R, 1);
+    PASS_LAUNCH(fluid_beside() <= PC_LANES_MAX, G, k_pc_apply, P, V, R, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT2, tape->m2, V.mrps, dyn);
     const bool reb = P.vapor_rebalance > 0.0f && has_vapor;
     if (reb) {
-      PASS_LAUNCH(crowded(loaded_fluid) <= PASS_LANES_MAX, pass_blocks(), k_rebalance1, P, V, 1);
+      PASS_LAUNCH(fluid_beside() <= PASS_LANES_MAX, pass_blocks(), k_rebalance1, P, V, 1);
       slab_point(SLAB_HALO, d);
     }
     LAUNCH(k_rebalance2_mark, G, kBlock, P, V, R, split_flag, reb ? 1 : 0, 1);

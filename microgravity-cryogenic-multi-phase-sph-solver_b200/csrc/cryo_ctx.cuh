@@ -443,9 +443,19 @@ struct cryo_ctx {
   // otherwise be idle.  Both shapes give the same bits, so a tank steps alike
   // alone and in an ensemble.  The rate passes have lanes in the exact
   // arithmetic only (cryo_lanes.cu), the phase-change passes always.
-  int crowd = 0;  // while an ensemble captures: the particles of the tanks side by side
-  int crowded(int own) const { return std::max(own, crowd); }
-  bool rate_lanes(int count, int most) const { return !fast_fields && P.use_lists && crowded(count) <= most; }
+  struct Crowd {
+    int fluid = 0, walls = 0;
+  } crowd;  // while an ensemble captures: the particles of the tanks side by side
+  int fluid_beside() const { return std::max(loaded_fluid, crowd.fluid); }
+  bool rate_lanes(int count, int most) const { return !fast_fields && P.use_lists && count <= most; }
+  bool list_lanes() const {
+    return loaded_n <= LIST_LANES_MAX &&
+           crowd.fluid + crowd.walls <= (P.has_vapor ? LIST_LANES_MAX_BESIDE : LIST_LANES_MAX_BESIDE_LIQUID);
+  }
+  bool wall_lanes() const {
+    return rate_lanes(loaded_n - loaded_fluid, P.has_vapor ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID) &&
+           crowd.walls <= (P.has_vapor ? WALL_LANES_MAX_BESIDE : WALL_LANES_MAX_BESIDE_LIQUID);
+  }
   int lane_blocks(int block = kBlock) const {
     const int per_block = block / PASS_LANES * grid_tile;
     return std::max(1, std::min((span() + per_block - 1) / per_block, sm_count * 64));

@@ -89,11 +89,15 @@ struct cryo_ensemble {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int launches = 0;
-    // fluid particles of the tanks that step side by side: the branches' share
-    long long fluid = 0;
-    for (const cryo_ctx* c : tanks) fluid += c->loaded_fluid;
-    const int crowd =
-        (int)std::min<long long>(fluid * branches() / std::max<long long>((long long)tanks.size(), 1), 1 << 30);
+    // particles of the tanks that step side by side: the branches' share
+    long long fluid = 0, walls = 0;
+    for (const cryo_ctx* c : tanks) {
+      fluid += c->loaded_fluid;
+      walls += c->loaded_n - c->loaded_fluid;
+    }
+    const long long share = std::max<long long>((long long)tanks.size(), 1);
+    const cryo_ctx::Crowd crowd{(int)std::min<long long>(fluid * branches() / share, 1 << 29),
+                                (int)std::min<long long>(walls * branches() / share, 1 << 29)};
     try {
       CK(cudaEventRecord(fork, stream));
       for (const auto& br : branches_plan) {
@@ -107,7 +111,7 @@ struct cryo_ensemble {
             int saved;
             ~TileScope() {
               c->grid_tile = saved;
-              c->crowd = 0;
+              c->crowd = {};
             }
           } scope{c, c->grid_tile};
           c->grid_tile = tile;

@@ -298,11 +298,21 @@ constexpr int forces_min_blocks(int what) {
 // Neighbour-list build: LIST_LANES lanes per particle up to LIST_LANES_MAX
 // particles, one above (k_build_lists).  One thread against lanes, us: 42 / 39
 // at 37 k particles, 52 / 57 at 55 k, 50 / 47 at 60 k (free surface, twice the
-// walls), 60 / 74 at 85 k.
+// walls), 60 / 74 at 85 k.  In an ensemble other members' kernels fill the chip
+// meanwhile, and the members together may hold LIST_LANES_MAX_BESIDE (_LIQUID:
+// no vapour).  Step of all, one thread / lanes: two-phase tanks 282 / 270 at
+// 54 k, 398 / 395 at 86 k, 451 / 451 at 108 k, 519 / 528 at 129 k; dam breaks
+// 182 / 168 at 95 k, 213 / 197 at 126 k, 275 / 273 at 201 k, 315 / 319 at 224 k.
 constexpr int LIST_LANES = 4;
 constexpr int kListPad = 8;  // records the build may load beyond the last particle
 #ifndef LIST_LANES_MAX
 #define LIST_LANES_MAX 60000
+#endif
+#ifndef LIST_LANES_MAX_BESIDE
+#define LIST_LANES_MAX_BESIDE 110000
+#endif
+#ifndef LIST_LANES_MAX_BESIDE_LIQUID
+#define LIST_LANES_MAX_BESIDE_LIQUID 190000
 #endif
 // The neighbour passes that come in two shapes, one thread per particle and
 // PASS_LANES lanes per particle, take the second up to these counts (fluid
@@ -330,6 +340,10 @@ constexpr int kListPad = 8;  // records the build may load beyond the last parti
 // Akinci's model, which sums over every neighbour.  The force pass's line is
 // the step's: with lanes 280 -> 275 us at 48 400 fluid particles (free surface),
 // 419 -> 380 at 46 700 (two phases), but 288 -> 299 at 55 000 (free surface).
+// In an ensemble the wall pass has lines of its own (step of all, one thread /
+// lanes): two-phase tanks 246 / 241 at 30 000 walls together, 253 / 246 at
+// 34 800, 294 / 293 at 40 000, 366 / 389 at 58 000; dam breaks 156 / 152 at
+// 60 500, 181 / 179 at 78 000, 207 / 207 at 88 000, 198 / 203 at 100 000.
 constexpr int PASS_LANES = 8;
 constexpr int FORCES_LANED_BLOCK = 128;
 #ifndef FORCES_LANES_MAX
@@ -355,6 +369,12 @@ constexpr int FORCES_LANED_BLOCK = 128;
 #endif
 #ifndef WALL_LANES_MAX_LIQUID  // no vapour
 #define WALL_LANES_MAX_LIQUID 57000
+#endif
+#ifndef WALL_LANES_MAX_BESIDE
+#define WALL_LANES_MAX_BESIDE 38000
+#endif
+#ifndef WALL_LANES_MAX_BESIDE_LIQUID
+#define WALL_LANES_MAX_BESIDE_LIQUID 85000
 #endif
 
 // Points a pressure probe gives a warp each; more take a thread each.  A warp
