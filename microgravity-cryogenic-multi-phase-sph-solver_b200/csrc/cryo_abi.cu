@@ -215,7 +215,7 @@ void cryo_ctx::sort_and_gather(int src, int list_mode, bool reset_maxima) {
 }
 
 void cryo_ctx::build_lists(const View& V, int mode) {
-  if (list_lanes())
+  if (shapes().list)
     LAUNCH(k_build_lists<LIST_LANES>, list_blocks(LIST_LANES), kBlock, P, V, reduce(), mode);
   else
     LAUNCH(k_build_lists<1>, list_blocks(1), kBlock, P, V, reduce(), mode);
@@ -226,17 +226,15 @@ void cryo_ctx::build_lists(const View& V, int mode) {
 void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) {
   const int G = grid_blocks(), GP = pass_blocks();
   const View V = view(s);
+  const Shapes laned = shapes();
   if (maxima_reset) LAUNCH(k_begin_step, 1, 1, P, V, BEGIN_RATES);
-  if (rate_lanes(fluid_beside(), PASS_LANES_MAX)) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
+  if (laned.density) LAUNCH(lanes::k_density, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_density, GP, kBlock, P, V, 1);
   slab_point(SLAB_HALO, s);
-  if (wall_lanes()) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
+  if (laned.wall) LAUNCH(lanes::k_wall, lane_blocks(), kBlock, P, V);
   else FIELD_LAUNCH(k_wall, GP, kBlock, P, V);
   slab_point(SLAB_HALO, s);
-  const int interface_max = P.st_model == CRYO_ST_AKINCI ? INTERFACE_LANES_MAX_AKINCI
-                            : P.has_vapor                ? INTERFACE_LANES_MAX
-                                                         : INTERFACE_LANES_MAX_WALLS;
-  if (rate_lanes(fluid_beside(), interface_max)) {
+  if (laned.interface) {
     if (tape) LAUNCH(lanes::k_interface<1>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
     else LAUNCH(lanes::k_interface<0>, lane_blocks(INTERFACE_BLOCK), INTERFACE_BLOCK, P, V, sorted ? 1 : 0);
   } else {
@@ -255,7 +253,6 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
     slab_point(SLAB_HALO, s);
   }
   const int GF = forces_blocks();
-  const bool laned = rate_lanes(fluid_beside(), FORCES_LANES_MAX);
   const int GL = lane_blocks(FORCES_LANED_BLOCK);
   // The instances with the rarer options compiled out (cryo_physics.cu).  In
   // the fast arithmetic only four sets have one: those where every sum is known
@@ -271,7 +268,7 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
   // such a window is in the exact arithmetic)
 #define FORCES_CASE(W)                                                       \
   case W:                                                                    \
-    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);   \
+    if (laned.forces) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);   \
     else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);             \
     break;
   if (tape) {
@@ -286,13 +283,13 @@ void cryo_ctx::evaluate_rates(int s, bool maxima_reset, bool sorted, bool tape) 
   }
 #define FORCES_CASE_COMMON(W)                                                                  \
   case W:                                                                                      \
-    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
+    if (laned.forces) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
     else if (common) FIELD_LAUNCH(k_forces_t<(W) | FORCE_COMMON>, GF, FORCES_BLOCK, P, V, W);  \
     else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);                               \
     break;
 #define FORCES_CASE_COMMON_EXACT(W)                                                            \
   case W:                                                                                      \
-    if (laned) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
+    if (laned.forces) LAUNCH(lanes::k_forces_t<W>, GL, FORCES_LANED_BLOCK, P, V);                     \
     else if (common && !fast_fields)                                                           \
       LAUNCH(exact::k_forces_t<(W) | FORCE_COMMON>, GF, FORCES_BLOCK, P, V, W);                \
     else FIELD_LAUNCH(k_forces_t<W>, GF, FORCES_BLOCK, P, V, W);                               \
@@ -368,15 +365,16 @@ void cryo_ctx::enqueue_step(int s, const StepTape* tape) {
   }
   if (P.cfg_phase_change) {
     const Reduce R = reduce();
-    PASS_LAUNCH(fluid_beside() <= PC_LANES_MAX, pass_blocks(), k_pc_normalize, P, V, 1);
+    const Shapes laned = shapes();
+    PASS_LAUNCH(laned.pc, pass_blocks(), k_pc_normalize, P, V, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.pc, tape->pc2, nullptr, nullptr, dyn);
-    PASS_LAUNCH(fluid_beside() <= PC_LANES_MAX, G, k_pc_apply, P, V, R, 1);
+    PASS_LAUNCH(laned.pc, G, k_pc_apply, P, V, R, 1);
     slab_point(SLAB_HALO, d);
     if (tape) LAUNCH(k_adj_copy4, G, kBlock, V.vT, tape->vT2, tape->m2, V.mrps, dyn);
     const bool reb = P.vapor_rebalance > 0.0f && has_vapor;
     if (reb) {
-      PASS_LAUNCH(fluid_beside() <= PASS_LANES_MAX, pass_blocks(), k_rebalance1, P, V, 1);
+      PASS_LAUNCH(laned.rebalance, pass_blocks(), k_rebalance1, P, V, 1);
       slab_point(SLAB_HALO, d);
     }
     LAUNCH(k_rebalance2_mark, G, kBlock, P, V, R, split_flag, reb ? 1 : 0, 1);
@@ -1750,6 +1748,14 @@ int cryo_load_state(cryo_ctx* c, const void* blob, size_t bytes) {
     c->has_vapor = h.has_vapor != 0;
     c->lists_built = false;
     CK(cudaMemcpyAsync(c->cell_begin, p, cells, cudaMemcpyHostToDevice, c->stream));
+    // the restored particles decide the passes' shapes, as a load's do
+    const unsigned old_shapes = c->shapes().bits();
+    const char* xp = static_cast<const char*>(blob) + sizeof(Blob);
+    int fluid = 0;
+    for (size_t i = 0; i < n; ++i) fluid += is_fluid(static_cast<unsigned char>(xp[16 * i + 12]));
+    c->loaded_n = (int)n;
+    c->loaded_fluid = fluid;
+    if (c->shapes().bits() != old_shapes || (c->grid_span > 0 && (int)n > c->span())) c->invalidate_graphs();
     c->sync();
   });
 }

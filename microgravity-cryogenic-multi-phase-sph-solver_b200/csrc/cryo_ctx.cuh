@@ -206,7 +206,7 @@ struct cryo_ctx {
   // solver state on the host side
   bool has_particles = false, initialized = false, has_vapor = false;
   bool lists_built = false;  // the neighbour lists of the current particles exist
-  int loaded_n = -1;  // particle count of the last set_particles / build_tank
+  int loaded_n = -1;  // particle count of the last set_particles / build_tank / load_state
   int loaded_fluid = 0;  // the liquid and vapour particles among them
   float char_length = 0;
   float pass_dt = 0;
@@ -446,15 +446,28 @@ struct cryo_ctx {
   struct Crowd {
     int fluid = 0, walls = 0;
   } crowd;  // while an ensemble captures: the particles of the tanks side by side
-  int fluid_beside() const { return std::max(loaded_fluid, crowd.fluid); }
-  bool rate_lanes(int count, int most) const { return !fast_fields && P.use_lists && count <= most; }
-  bool list_lanes() const {
-    return loaded_n <= LIST_LANES_MAX &&
-           crowd.fluid + crowd.walls <= (P.has_vapor ? LIST_LANES_MAX_BESIDE : LIST_LANES_MAX_BESIDE_LIQUID);
-  }
-  bool wall_lanes() const {
-    return rate_lanes(loaded_n - loaded_fluid, P.has_vapor ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID) &&
-           crowd.walls <= (P.has_vapor ? WALL_LANES_MAX_BESIDE : WALL_LANES_MAX_BESIDE_LIQUID);
+  struct Shapes {  // true: with lanes
+    bool list, density, wall, interface, forces, pc, rebalance;
+    unsigned bits() const {
+      return list | density << 1 | wall << 2 | interface << 3 | forces << 4 | pc << 5 | rebalance << 6;
+    }
+  };
+  Shapes shapes() const {
+    const int fluid = std::max(loaded_fluid, crowd.fluid), walls = loaded_n - loaded_fluid;
+    const bool rate = !fast_fields && P.use_lists, vapour = P.has_vapor != 0;
+    Shapes s;
+    s.list = loaded_n <= LIST_LANES_MAX &&
+             crowd.fluid + crowd.walls <= (vapour ? LIST_LANES_MAX_BESIDE : LIST_LANES_MAX_BESIDE_LIQUID);
+    s.density = rate && fluid <= PASS_LANES_MAX;
+    s.wall = rate && walls <= (vapour ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID) &&
+             crowd.walls <= (vapour ? WALL_LANES_MAX_BESIDE : WALL_LANES_MAX_BESIDE_LIQUID);
+    s.interface = rate && fluid <= (P.st_model == CRYO_ST_AKINCI ? INTERFACE_LANES_MAX_AKINCI
+                                    : vapour                     ? INTERFACE_LANES_MAX
+                                                                 : INTERFACE_LANES_MAX_WALLS);
+    s.forces = rate && fluid <= FORCES_LANES_MAX;
+    s.pc = fluid <= PC_LANES_MAX;
+    s.rebalance = fluid <= PASS_LANES_MAX;
+    return s;
   }
   int lane_blocks(int block = kBlock) const {
     const int per_block = block / PASS_LANES * grid_tile;
