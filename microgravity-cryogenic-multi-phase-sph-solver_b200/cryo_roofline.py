@@ -60,8 +60,8 @@ def per_particle(kernel: str, cfg, has_vapor: bool):
         return fl, 1 + (13 if f["pc"] else 0)
     if kernel == "k_saturation":
         return 9, 1
-    if kernel == "k_cell_scatter":  # key in; place drawn: old index and key out
-        return 4 + 4 + 4, 4 + 4 + 4
+    if kernel == "k_cell_scatter":  # key and number drawn in; old index and key out
+        return 16, 16
     if kernel == "k_cell_order":  # key and old index in; permutation out
         return 12, 12
     if kernel == "k_cells":  # a table filled from sorted keys
@@ -71,8 +71,9 @@ def per_particle(kernel: str, cfg, has_vapor: bool):
 
 def kernel_bytes(kernel: str, cfg, n_fluid: int, n_wall: int, has_vapor: bool, num_cells: int = 0) -> float:
     fl, wl = per_particle(kernel, cfg, has_vapor)
-    # per cell: the table out; the scan also reads the counts
-    extra = {"k_cells": 4, "k_cell_scan": 8}.get(kernel, 0) * (num_cells + 1)
+    # per cell.  k_cells: the table out.  Scan: count in, its zero, the prefix
+    # and the cleared kinds out.  Scatter: prefix in, table out.  Order: table in.
+    extra = {"k_cells": 4, "k_cell_scan": 16, "k_cell_scatter": 8, "k_cell_order": 4}.get(kernel, 0) * (num_cells + 1)
     return float(fl * n_fluid + wl * n_wall + extra)
 
 

@@ -274,10 +274,15 @@ constexpr int FORCE_BASE = FORCE_TRANSPORT | FORCE_MOMENTUM | FORCE_MAXIMA;
 #ifndef FORCES_MIN_BLOCKS
 #define FORCES_MIN_BLOCKS 9
 #endif
-// The sub-pass sets with surface tension or heat run without spilling at 8
-// blocks per SM (4 warps per sub-partition); the instances with FORCE_COMMON
-// fit 10: 778 us against 874 at 1.06 M particles in the fast arithmetic, 3619
-// against 3842 at 4.08 M in the exact one.  At 12 they spill (963 and 4599 us).
+// The sub-pass sets with surface tension or heat take 8 blocks per SM (4 warps
+// per sub-partition, 128 registers); the instances with FORCE_COMMON 10 (96):
+// 778 us against 874 at 1.06 M particles in the fast arithmetic, 3619 against
+// 3842 at 4.08 M in the exact one.  Some of them spill 4-48 bytes at 10 (the
+// exact sets with the density rate, and the fast CSF with heat) and are still
+// ahead of their general instances at 8: CSF with heat and density rate 1027 us
+// against 1270 at 729 k fluid particles, CSF with density rate 972 against
+// 1181, heat with density rate 709 against 841 at 405 k.  At 12 they spill more
+// (963 and 4599 us).
 #ifndef FORCES_MIN_BLOCKS_HEAVY
 #define FORCES_MIN_BLOCKS_HEAVY 8
 #endif
@@ -290,8 +295,7 @@ constexpr int forces_min_blocks(int what) {
                                                               : FORCES_MIN_BLOCKS_HEAVY;
 }
 // Neighbour-loop unroll of the force-pass variants with surface tension or
-// heat (the two-phase tanks): 2 takes the 4 M-particle LH2 sphere 3 % faster,
-// no spills.
+// heat (the two-phase tanks): 2 takes the 4 M-particle LH2 sphere 3 % faster.
 #ifndef FORCES_UNROLL_HEAVY
 #define FORCES_UNROLL_HEAVY 2
 #endif

@@ -365,18 +365,14 @@ __global__ void __launch_bounds__(kBlock) k_smooth_normals(Params P, View V) {
   }
 }
 
-// Fused force pass: compute_transport_acceleration (SPH_kernels.cu:56-104),
-// compute_momentum (navier_stokes.cu:121-245), apply_csf_surface_tension
-// (surface_tension.cu:120-177) or apply_akinci_surface_tension (:179-213),
-// compute_density_rate (SPH_kernels.cu:162-203), compute_thermal_rates
-// (phase_change.cu:31-75) and the dt maxima (sph_solver.cu:59-99, 475-479),
-// in one neighbour loop.  Each sub-pass reads only what the previous passes
-// wrote, never what this pass writes, so fusing keeps the reference's values.
 // Vi^2 + Vj^2 with Vi2 = Vi^2.  In the fast arithmetic the compiler contracts
 // it into either product, differently from one instance of the force pass to
-// the next; the instances with FORCE_COMMON state it (FMA 1: the neighbour's
-// square is the fused one, 2: the particle's own), so that a particle's sums
-// keep the bits of the general instance.
+// the next; the instances with FORCE_COMMON state the form the general instance
+// of their set has (FMA 1: the neighbour's square is the fused one, 2: the
+// particle's own).  A configuration only ever runs one of the two, so nothing
+// rests on their bits being equal: they are, with nvcc 12.9, with lists, without
+// and for more neighbours than a list holds, and another compiler may move the
+// last bit of either within the fast arithmetic's bounds.
 template <int FMA>
 __device__ inline float sum_squares(float Vi, float Vi2, float Vj) {
   if (FMA == 1) return __fmaf_rn(Vj, Vj, Vi2);
@@ -384,13 +380,6 @@ __device__ inline float sum_squares(float Vi, float Vi2, float Vj) {
   return Vi2 + Vj * Vj;
 }
 
-// FORCE_COMMON instances: Wendland kernel, no sub-particle stresses, no
-// transport stress, plain CSF, walls not isothermal, known when compiled.  The
-// pass issues instructions all the time (two thirds of its issue slots, DRAM a
-// tenth busy), and each of those options cost a test per pair and registers
-// over the whole loop: without them 4.08 M particles took 4024 us in place of
-// 4718, 1.06 M in the fast arithmetic 778 in place of 1018, the dam of 204 k
-// 128 in place of 152.
 // A sum of the force pass that few pairs add to (walls, the interface): in
 // registers, or in a column of shared memory that leaves them free over every
 // pair.  With the columns the exact pass of a two-phase tank fits 96 registers
@@ -412,6 +401,22 @@ struct SumV3<true> {
   __device__ void set(V3 v) { p[0] = v.x; p[FORCES_BLOCK] = v.y; p[2 * FORCES_BLOCK] = v.z; }
   __device__ void operator+=(V3 a) { V3 s = get(); s += a; set(s); }
 };
+
+// Fused force pass: compute_transport_acceleration (SPH_kernels.cu:56-104),
+// compute_momentum (navier_stokes.cu:121-245), apply_csf_surface_tension
+// (surface_tension.cu:120-177) or apply_akinci_surface_tension (:179-213),
+// compute_density_rate (SPH_kernels.cu:162-203), compute_thermal_rates
+// (phase_change.cu:31-75) and the dt maxima (sph_solver.cu:59-99, 475-479),
+// in one neighbour loop.  Each sub-pass reads only what the previous passes
+// wrote, never what this pass writes, so fusing keeps the reference's values.
+//
+// FORCE_COMMON instances: Wendland kernel, no sub-particle stresses, no
+// transport stress, plain CSF, walls not isothermal, known when compiled.  The
+// pass issues instructions all the time (two thirds of its issue slots, DRAM a
+// tenth busy), and each of those options cost a test per pair and registers
+// over the whole loop: without them 4.08 M particles took 4024 us in place of
+// 4718, 1.06 M in the fast arithmetic 778 in place of 1018, the dam of 204 k
+// 128 in place of 152.
 template <int WHAT>
 __global__ void __launch_bounds__(FORCES_BLOCK, forces_min_blocks(WHAT)) k_forces_t(Params P, View V, int what_rt) {
   // WHAT >= 0: the sub-pass set is a compile-time constant (the step path);

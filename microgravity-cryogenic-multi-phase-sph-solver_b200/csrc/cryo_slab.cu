@@ -84,7 +84,8 @@ __global__ void __launch_bounds__(kBlock) k_halo_pull(Params P, View dst, View s
 }
 
 // Heat-weight normalisation over every slab (sph_solver.cu:466-472): the
-// owned sums added in slab order.  heat_mode is the pass's heat_sum switch.
+// owned sums added in slab order.  heat_mode 2:
+// also while heat is off.
 __global__ void k_slab_heat(Params P, DynState* const* dyns, int nslabs, DynState* mine, int heat_mode) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   double S = 0.0;
