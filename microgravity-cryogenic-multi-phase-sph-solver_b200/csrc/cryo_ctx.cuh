@@ -445,7 +445,7 @@ struct cryo_ctx {
   // arithmetic only (cryo_lanes.cu), the phase-change passes always.
   struct Crowd {
     int fluid = 0, walls = 0;
-  } crowd;  // while an ensemble captures: the particles of the tanks side by side
+  } crowd;  // the particles of the tanks side by side, while an ensemble captures; of the slabs of one device
   struct Shapes {  // true: with lanes
     bool list, density, wall, interface, forces, pc, rebalance;
     unsigned bits() const {

@@ -554,6 +554,23 @@ int cryo_slabs_set_particles(cryo_slabs* s, const cryo_host_particles_t* p, cons
       c->finish_load(m, next_id);
       G.alloc_spare(r);
     }
+    // slabs of one device step side by side: their passes choose by the
+    // particles they own together (the passes skip the ghosts)
+    std::vector<cryo_ctx::Crowd> own(R);
+    for (int i = 0; i < n; ++i) {
+      const int r = (int)(std::upper_bound(G.zb.begin(), G.zb.end(), layer[i]) - G.zb.begin()) - 1;
+      if (r >= 0 && r < R) ++(is_fluid(p->phase[i]) ? own[r].fluid : own[r].walls);
+    }
+    for (cryo_ctx* c : G.slabs) {
+      const unsigned old_shapes = c->shapes().bits();
+      c->crowd = {};
+      for (int q = 0; R > 1 && q < R; ++q)
+        if (G.slabs[q]->device == c->device) {
+          c->crowd.fluid += own[q].fluid;
+          c->crowd.walls += own[q].walls;
+        }
+      if (c->shapes().bits() != old_shapes) c->invalidate_graphs();
+    }
   });
 }
 
