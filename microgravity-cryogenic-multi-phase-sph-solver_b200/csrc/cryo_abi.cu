@@ -1748,11 +1748,15 @@ int cryo_load_state(cryo_ctx* c, const void* blob, size_t bytes) {
     c->has_vapor = h.has_vapor != 0;
     c->lists_built = false;
     CK(cudaMemcpyAsync(c->cell_begin, p, cells, cudaMemcpyHostToDevice, c->stream));
-    // the restored particles decide the passes' shapes, as a load's do
+    // the restored particles decide the passes' shapes, as a load's do; a state
+    // that has been sorted holds its counts
     const unsigned old_shapes = c->shapes().bits();
-    const char* xp = static_cast<const char*>(blob) + sizeof(Blob);
-    int fluid = 0;
-    for (size_t i = 0; i < n; ++i) fluid += is_fluid(static_cast<unsigned char>(xp[16 * i + 12]));
+    int fluid = std::max(0, (int)n - h.dyn.n_wall_list);
+    if (!h.initialized) {
+      const char* xp = static_cast<const char*>(blob) + sizeof(Blob);
+      fluid = 0;
+      for (size_t i = 0; i < n; ++i) fluid += is_fluid(static_cast<unsigned char>(xp[16 * i + 12]));
+    }
     c->loaded_n = (int)n;
     c->loaded_fluid = fluid;
     if (c->shapes().bits() != old_shapes || (c->grid_span > 0 && (int)n > c->span())) c->invalidate_graphs();

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 DX = 0.004
 
 
-def solver(layers):
+def solver(layers, steps=2):
     """The lower layers of a box of 110 592 fluid particles, in the whole box's domain."""
     water = cs.FluidProperties.water()
     box = cs.BoxTank(48 * DX, 48 * DX, 48 * DX)
@@ -28,7 +28,8 @@ def solver(layers):
     lo, hi = cs.tank_domain(box, DX, 3)
     s.set_particles(q["position"], q["mass"], q["density"], q["temperature"], q["phase"], domain_lo=lo, domain_hi=hi,
                     normal=q["normal"], flags=q["flags"])
-    s.run_steps(2)
+    if steps:
+        s.run_steps(steps)
     return s
 
 
@@ -57,3 +58,11 @@ def test_restored_state_chooses_the_shapes(cuda_device, graph):
     a, b = small.particles(), large.particles()
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+def test_state_saved_before_the_first_step(cuda_device):
+    """A state that has not been sorted is counted."""
+    small, large = solver(4, 0), solver(48, 0)
+    blob = large.save_state()
+    small.load_state(blob)
+    assert kernels(small) == {"threads"}
