@@ -456,8 +456,7 @@ struct cryo_ctx {
     const int fluid = std::max(loaded_fluid, crowd.fluid), walls = loaded_n - loaded_fluid;
     const bool rate = !fast_fields && P.use_lists, vapour = P.has_vapor != 0;
     Shapes s;
-    s.list = loaded_n <= LIST_LANES_MAX &&
-             crowd.fluid + crowd.walls <= (vapour ? LIST_LANES_MAX_BESIDE : LIST_LANES_MAX_BESIDE_LIQUID);
+    s.list = loaded_n <= LIST_LANES_MAX && crowd.fluid <= LIST_LANES_MAX_BESIDE;
     s.density = rate && fluid <= PASS_LANES_MAX;
     s.wall = rate && walls <= (vapour ? WALL_LANES_MAX : WALL_LANES_MAX_LIQUID) &&
              crowd.walls <= (vapour ? WALL_LANES_MAX_BESIDE : WALL_LANES_MAX_BESIDE_LIQUID);

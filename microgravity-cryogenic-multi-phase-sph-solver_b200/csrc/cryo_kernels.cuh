@@ -303,20 +303,19 @@ constexpr int forces_min_blocks(int what) {
 // particles, one above (k_build_lists).  One thread against lanes, us: 42 / 39
 // at 37 k particles, 52 / 57 at 55 k, 50 / 47 at 60 k (free surface, twice the
 // walls), 60 / 74 at 85 k.  In an ensemble other members' kernels fill the chip
-// meanwhile, and the members together may hold LIST_LANES_MAX_BESIDE (_LIQUID:
-// no vapour).  Step of all, one thread / lanes: two-phase tanks 282 / 270 at
-// 54 k, 398 / 395 at 86 k, 451 / 451 at 108 k, 519 / 528 at 129 k; dam breaks
-// 182 / 168 at 95 k, 213 / 197 at 126 k, 275 / 273 at 201 k, 315 / 319 at 224 k.
+// meanwhile, and the members together may hold LIST_LANES_MAX_BESIDE fluid
+// particles (a wall's list is short, so the fluid sets the work).  Step of all,
+// one thread / lanes, exact and fast, by fluid particles together: two-phase
+// tanks 32 k 323 / 315 and 380 / 385, 47 k 451 / 450 and 444 / 447, 55 k 572 /
+// 586 and 522 / 518, 59 k 480 / 492 and 439 / 455; dam breaks 34 k 275 / 273 and
+// 319 / 310, 53 k 360 / 360 and 345 / 344, 65 k 354 / 373 and 348 / 361.
 constexpr int LIST_LANES = 4;
 constexpr int kListPad = 8;  // records the build may load beyond the last particle
 #ifndef LIST_LANES_MAX
 #define LIST_LANES_MAX 60000
 #endif
 #ifndef LIST_LANES_MAX_BESIDE
-#define LIST_LANES_MAX_BESIDE 110000
-#endif
-#ifndef LIST_LANES_MAX_BESIDE_LIQUID
-#define LIST_LANES_MAX_BESIDE_LIQUID 190000
+#define LIST_LANES_MAX_BESIDE 56000
 #endif
 // The neighbour passes that come in two shapes, one thread per particle and
 // PASS_LANES lanes per particle, take the second up to these counts (fluid
