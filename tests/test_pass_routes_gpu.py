@@ -91,7 +91,10 @@ def shapes_of(run):
     torch.zeros(1, device="cuda")
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         run()
-    return {e.key for e in prof.key_averages()}
+    names = {e.key for e in prof.key_averages()}
+    if not any("k_" in k for k in names):
+        pytest.skip("the profiler records no kernels here")
+    return names
 
 
 def test_an_ensemble_changes_the_shapes_and_no_bit(cuda_device):
@@ -119,6 +122,9 @@ def test_an_ensemble_changes_the_shapes_and_no_bit(cuda_device):
     crowd.add(beside)
     alone.run_steps(6)
     crowd.run_steps(6)
+    a, b = alone.particles(), beside.particles()
+    same(a, b)
+    assert alone.diagnostics().as_dict() == beside.diagnostics().as_dict()
     with_lanes = shapes_of(lambda: (alone.run_steps(2), alone.diagnostics()))
     with_threads = shapes_of(lambda: (crowd.run_steps(2), crowd.diagnostics()))
     for name, lanes, threads in (("k_density", "lanes::", "exact::"), ("k_wall", "lanes::", "exact::"),
@@ -129,9 +135,6 @@ def test_an_ensemble_changes_the_shapes_and_no_bit(cuda_device):
         b = [k for k in with_threads if name in k]
         assert a and all(lanes in k and threads not in k for k in a), (name, a)
         assert b and all(threads in k and lanes not in k for k in b), (name, b)
-    a, b = alone.particles(), beside.particles()
-    same(a, b)
-    assert alone.diagnostics().as_dict() == beside.diagnostics().as_dict()
 
 
 @pytest.mark.parametrize("base,other", [(b, o) for b, o, arithmetics in OTHER_ROUTE if 1 in arithmetics])

@@ -39,7 +39,10 @@ def kernels(s):
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         s.step()
         s.diagnostics()
-    return {"lanes" if "lanes::" in e.key else "threads" for e in prof.key_averages() if "k_forces_t" in e.key}
+    names = {e.key for e in prof.key_averages()}
+    if not any("k_" in k for k in names):
+        pytest.skip("the profiler records no kernels here")
+    return {"lanes" if "lanes::" in k else "threads" for k in names if "k_forces_t" in k}
 
 
 @pytest.mark.parametrize("graph", [False, True])
